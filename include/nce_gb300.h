@@ -171,7 +171,8 @@ typedef struct {
     int32_t ex_parity;         /* used when ex_u != NULL */
     const double *ex_u;        /* (ceil((R-1)/2)) device uniforms, or NULL -> Philox */
     int32_t precision;         /* 64 or 32 */
-    int32_t warps;             /* warps per replica (0 = default) */
+    int32_t warps;             /* warps per replica (0 = default); the windowed sign-parity kernel (one basis site per
+                                  cell) has a launch shape of its own and ignores warps and cluster */
     int32_t path;              /* 0 auto (local field when the state has a field, else sign parity when the point
                                   functions are in {-1,+1}, else general), 1 general point-function products, 2 sign
                                   parity, 3 local field (precision 64, state.field set) */

@@ -15,7 +15,9 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <array>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -30,6 +32,7 @@ namespace cg = cooperative_groups;
 namespace nce {
 
 constexpr int kMaxJobs = 64;
+struct WinTab;                           // tables of the windowed kernel (ce_window.cuh)
 
 struct CEJob {
     // tables (device)
@@ -84,6 +87,7 @@ struct CEJob {
     int32_t *rep_of_slot; const int32_t *ladder_id; int64_t *n_ex; const double *ex_u;
     int32_t *ex_sync;      // replicas of the job done with the chunk (0 between chunks)
     int32_t ex_flags;      // bit 0: the chunk ends on an exchange; bit 1: host parity (with ex_u)
+    const WinTab *win;     // windowed kernel
 };
 
 struct CEBatch {
@@ -1173,6 +1177,8 @@ __global__ void __launch_bounds__(32 * kLfMaxWarps) ce_lf_chunk_kernel(const __g
     if (warp == 0 && jb.ex_sync) fused_chunk_end(jb, g0, lane);
 }
 
+#include "ce_window.cuh"
+
 // Full energy on the sign-parity tables, bit-sliced.  The occupancies become bit planes: per replica, point-
 // function column with sign changes and basis site, one row of 2 * d2 bits per (k0, k1) holding the sign bit of
 // every k2 twice over, so that any offset in [0, d2) reads 32 consecutive bits with one funnel shift.  A thread
@@ -1514,6 +1520,11 @@ struct nce_ce_model {
     int32_t *lf_off = nullptr; uint16_t *lf_idx = nullptr; int16_t *lf_box = nullptr;
     int32_t lf_e[3] = {0, 0, 0}, lf_nidx = 0;
     uint32_t *frows = nullptr; int4 *fmem = nullptr; int32_t *frow_off = nullptr, *frow_n = nullptr;
+    // windowed kernel: host copy of the table header (device pointers inside) and its device copy, null when the cell
+    // or the cluster set cannot use it
+    nce::WinTab win_host; nce::WinTab *win = nullptr;
+    int4 *win_ent = nullptr; uint32_t *win_desc = nullptr; uint2 *win_seg = nullptr; int32_t *win_seg_off = nullptr;
+    int16_t *win_nbr = nullptr, *win_alias = nullptr; int32_t *win_csign = nullptr;
 
     int device = 0;
     std::mutex mu;
@@ -1534,7 +1545,8 @@ static int upload(T *&dst, const T *src, size_t n) {
 static int free_model(nce_ce_model *m) {
     void *ptrs[] = {m->loc, m->pfc, m->eci64, m->eci32, m->rv_len, m->nb_b, m->nb_uo, m->pf64, m->pf32, m->act_b,
                     m->act_nb, m->grp_cum, m->T_b, m->T_uo, m->T_pfc, m->T_eci64, m->T_eci32, m->err, m->sbits, m->bix, m->rcol, m->ecol2_64, m->ecol2_32, m->ecol_fix, m->chunks, m->n_chunks, m->brows, m->bmem, m->brow_off, m->brow_n, m->plane_pfc, m->ecol1,
-                    m->staging_base, m->lf_off, m->lf_idx, m->lf_box, m->frows, m->fmem, m->frow_off, m->frow_n};
+                    m->staging_base, m->lf_off, m->lf_idx, m->lf_box, m->frows, m->fmem, m->frow_off, m->frow_n,
+                    m->win, m->win_ent, m->win_desc, m->win_seg, m->win_seg_off, m->win_nbr, m->win_alias, m->win_csign};
     for (void *p : ptrs) if (p) cudaFree(p);
     delete m;
     return NCE_OK;
@@ -1579,6 +1591,7 @@ static CEJob make_job(const nce_ce_model *m, const nce_pt_state *st, const nce_p
         j.ex_u = ck->ex_u; j.ex_flags = (ck->do_exchange ? 1 : 0) | ((ck->ex_parity & 1) << 1);
         j.lf_off = m->lf_off; j.lf_idx = m->lf_idx; j.lf_box = m->lf_box;
         j.lf_e0 = m->lf_e[0]; j.lf_e1 = m->lf_e[1]; j.lf_e2 = m->lf_e[2]; j.lf_nidx = m->lf_nidx;
+        j.win = m->win;
         j.near_eV = ck->near_eV > 0.0 ? ck->near_eV : (p64 ? 1e-9 : 1e-6);
         if (j.fix_shift > 0) {
             const double nf = std::ldexp(j.near_eV, j.fix_shift);
@@ -1652,6 +1665,15 @@ static int launch_lf(const CEBatch &bt, int mo, int total, int warps, size_t sme
     }
     NCE_CUDA(::nce::raise_smem_limit((const void *)kern, smem));
     kern<<<total, std::min(warps, kLfMaxWarps) * 32, smem, s>>>(bt, budget);
+    NCE_CUDA(cudaGetLastError());
+    return NCE_OK;
+}
+
+template <typename Acc>
+static int launch_win(const CEBatch &bt, int total, int threads, size_t smem, cudaStream_t s) {
+    auto kern = ce_win_chunk_kernel<Acc>;
+    NCE_CUDA(::nce::raise_smem_limit((const void *)kern, smem));
+    kern<<<total, threads, smem, s>>>(bt);
     NCE_CUDA(cudaGetLastError());
     return NCE_OK;
 }
@@ -1745,7 +1767,20 @@ static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *st
     size_t smem = 0; bool all_fit = true;
     int sig_smem = 0;
     int64_t lf_budget = 0;
-    if (use_lf) {
+    // windowed kernel wherever the sign-parity path runs and every job has its tables (build_window_tables): it was faster
+    // at every size and ladder measured, against the step-by-step kernel at its best launch shape (2,048 sites x 32
+    // replicas, 1,000 steps: 1,202 -> 281 us; 131,072 x 256, 300 steps: 1,196 -> 116 us; 256 x 16, 10 steps: 63 -> 26 us;
+    // 24 float32 jobs of 256 to 32,000 sites, 500 steps: 4,154 -> 759 us).  warps and cluster only shape the
+    // step-by-step kernels, which keep the other tables (several basis sites, larger orders, one-cell images).
+    bool use_win = use_bin;
+    for (int j = 0; j < n_jobs; ++j) use_win = use_win && hs[j]->win != nullptr;
+    constexpr int win_threads = 512;
+    if (use_win) {
+        for (int j = 0; j < n_jobs; ++j) {
+            const WinTab &w = hs[j]->win_host;
+            smem = std::max(smem, WinLayout::make(w.n_ent, w.n_blk, w.n_seg, hs[j]->n_cols).total);
+        }
+    } else if (use_lf) {
         size_t t_on = 0, t_off = 0; int64_t maxN = 0;
         for (int j = 0; j < n_jobs; ++j) {
             const nce_ce_model *m = hs[j];
@@ -1841,7 +1876,10 @@ static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *st
             // every CTA of a cluster keeps its own copy of the occupancy: all jobs must fit the shared-memory budget
             for (int j = 0; j < n_jobs; ++j) if (!bt.job[j].sig_smem) CL = 1;
         }
-        if (use_lf)
+        if (use_win)
+            rc = precision == 64 ? launch_win<double>(bt, total, win_threads, smem, s)
+                                 : launch_win<float>(bt, total, win_threads, smem, s);
+        else if (use_lf)
             rc = launch_lf(bt, mo, total, warps, smem, (int32_t)lf_budget, s);
         else if (use_bin)
             rc = precision == 64 ? launch_bin<double>(bt, mo, total, warps, smem, sig_smem, s, CL)
@@ -2032,6 +2070,120 @@ static int build_local_field_tables(nce_ce_model *m, const nce_ce_tables *t, con
     return NCE_OK;
 }
 
+// Tables of the windowed kernel (ce_window.cuh), built when the set and the cell allow it: one basis site, two species
+// of opposite sign on one point-function column, at most three members beside the site in a row, no row that holds one
+// site twice (tiny cells), every column's rows of one order, and the reverse rows closed (an instance that a row lists is
+// listed by a row of each of its members: flipping b, then a, then counts every changed instance once).  Otherwise
+// m->win stays null and the step-by-step kernels run.
+static int build_window_tables(nce_ce_model *m, const nce_ce_tables *t, const std::vector<uint8_t> &sb) {
+    if (t->nB != 1 || t->max_sp != 2 || t->mo > 4 || t->n_groups != 1 || t->n_nbr > 1000 || t->J > 16000) return NCE_OK;
+    const int mo = t->mo, n_nbr = t->n_nbr, n_rows = t->Rv_len[0];
+    int real = -1;                                           // the point-function column that changes sign
+    for (int c = 0; c < t->n_pfc; ++c) {
+        if (sb[(size_t)c * 4] == 0 && sb[(size_t)c * 4 + 1] == 0) continue;
+        if (real >= 0 || sb[(size_t)c * 4] == sb[(size_t)c * 4 + 1]) return NCE_OK;
+        real = c;
+    }
+    if (real < 0) return NCE_OK;
+    WinTab w; std::memset(&w, 0, sizeof(w));
+    w.n_ent = n_nbr;
+    std::vector<int32_t> so((size_t)n_nbr * 3);              // signed offsets in (-d/2, d/2]
+    for (int c = 0; c < 3; ++c) {
+        int64_t lo = 0, hi = 0;
+        for (int n = 0; n < n_nbr; ++n) {
+            int64_t x = t->nb_uo[3 * n + c];
+            if (x > t->d[c] / 2) x -= t->d[c];
+            so[3 * n + c] = (int32_t)x;
+            lo = std::max(lo, -x); hi = std::max(hi, x);
+        }
+        w.lo[c] = (int32_t)lo; w.ext[c] = (int32_t)(lo + hi + 1);
+    }
+    if (m->N >= 2147483647ll || t->d[0] + t->d[1] + t->d[2] >= 1000000000ll) return NCE_OK;
+    const int64_t box = (int64_t)w.ext[0] * w.ext[1] * w.ext[2];
+    if (box > (1ll << 24)) return NCE_OK;
+    std::vector<int4> ent((size_t)n_nbr); std::vector<int16_t> nbr((size_t)box, (int16_t)-1), alias((size_t)n_nbr, (int16_t)-1);
+    for (int n = 0; n < n_nbr; ++n) {
+        const int32_t *x = &so[3 * n];
+        const int64_t i = ((int64_t)(x[0] + w.lo[0]) * w.ext[1] + (x[1] + w.lo[1])) * w.ext[2] + x[2] + w.lo[2];
+        ent[n] = make_int4(t->nb_uo[3 * n], t->nb_uo[3 * n + 1], t->nb_uo[3 * n + 2], (int32_t)i);
+        alias[n] = nbr[(size_t)i]; nbr[(size_t)i] = (int16_t)n;
+    }
+    if (t->nb_uo[0] || t->nb_uo[1] || t->nb_uo[2]) return NCE_OK;   // entry 0 is the site itself
+    // rows: the members beside the site, by column; instances by (column, sites relative to the member)
+    std::vector<int> order((size_t)t->n_cols, -1);
+    std::vector<std::vector<std::vector<int>>> by_col((size_t)t->n_cols);
+    std::map<std::vector<int32_t>, int> inst;                // instance seen from its site -> rows listed - rows implied
+    for (int q = 0; q < n_rows; ++q) {
+        std::vector<int> oth; int own = 0;
+        for (int k = 0; k < mo; ++k) {
+            if (t->Rv_pfc[(size_t)q * mo + k] != real) continue;
+            const int n = t->Rv_loc[(size_t)q * mo + k];
+            if (n == 0) ++own; else oth.push_back(n);
+        }
+        if (own != 1) return NCE_OK;
+        const int col = t->Rv_col[q], ord = (int)oth.size() + 1;
+        if (order[col] >= 0 && order[col] != ord) return NCE_OK;
+        order[col] = ord;
+        std::vector<std::array<int32_t, 3>> pts(1, {0, 0, 0});
+        for (int n : oth) pts.push_back({t->nb_uo[3 * n], t->nb_uo[3 * n + 1], t->nb_uo[3 * n + 2]});
+        for (size_t x = 0; x < pts.size(); ++x)
+            for (size_t y = 0; y < x; ++y) if (pts[x] == pts[y]) return NCE_OK;
+        for (size_t x = 0; x < pts.size(); ++x) {            // the same instance seen from each of its members
+            std::vector<std::array<int32_t, 3>> rel;
+            for (const auto &p : pts) {
+                std::array<int32_t, 3> z;
+                for (int c = 0; c < 3; ++c) { int64_t v = (int64_t)p[c] - pts[x][c]; z[c] = (int32_t)(v < 0 ? v + t->d[c] : v); }
+                rel.push_back(z);
+            }
+            std::sort(rel.begin(), rel.end());
+            std::vector<int32_t> key(1, col);
+            for (const auto &z : rel) key.insert(key.end(), z.begin(), z.end());
+            inst[key] += x == 0 ? ord - 1 : -1;
+        }
+        if (!oth.empty()) by_col[col].push_back(oth);
+    }
+    for (const auto &kv : inst) if (kv.second != 0) return NCE_OK;
+    // lanes: kWinRows rows of one column each, 32 lanes a block; a column's lanes within a block form one segment
+    std::vector<uint32_t> desc; std::vector<uint2> seg; std::vector<int32_t> seg_off(1, 0);
+    const uint32_t zero = (uint32_t)n_nbr * 4u, none = zero | (zero << 10) | (zero << 20);
+    int lane = 32;
+    for (int c = 0; c < t->n_cols; ++c)
+        for (size_t q = 0; q < by_col[c].size(); q += kWinRows) {
+            if (lane == 32) {
+                if (!desc.empty()) seg_off.push_back((int32_t)seg.size());
+                desc.resize(desc.size() + 32 * kWinRows, none); lane = 0;
+            }
+            uint32_t *d = &desc[desc.size() - 32 * kWinRows];
+            for (size_t h = 0; h < kWinRows && q + h < by_col[c].size(); ++h) {
+                uint32_t ix[3] = {zero, zero, zero};
+                for (size_t k = 0; k < by_col[c][q + h].size(); ++k) ix[k] = (uint32_t)by_col[c][q + h][k] * 4u;
+                d[h * 32 + lane] = ix[0] | (ix[1] << 10) | (ix[2] << 20);
+            }
+            if ((size_t)seg_off.back() < seg.size() && seg.back().y == (uint32_t)c) seg.back().x |= 1u << lane;
+            else seg.push_back(make_uint2(1u << lane, (uint32_t)c));
+            ++lane;
+        }
+    if (desc.empty()) return NCE_OK;
+    seg_off.push_back((int32_t)seg.size());
+    w.n_blk = (int32_t)seg_off.size() - 1; w.n_seg = (int32_t)seg.size();
+    if (WinLayout::make(w.n_ent, w.n_blk, w.n_seg, t->n_cols).total > 96 * 1024) return NCE_OK;
+    std::vector<int32_t> csign((size_t)t->n_cols, 2);
+    for (int c = 0; c < t->n_cols; ++c) if (sb[(size_t)real * 4] && (order[c] & 1) && order[c] > 0) csign[c] = -2;
+    int rc = upload(m->win_ent, ent.data(), ent.size());
+    if (!rc) rc = upload(m->win_desc, desc.data(), desc.size());
+    if (!rc) rc = upload(m->win_seg, seg.data(), seg.size());
+    if (!rc) rc = upload(m->win_seg_off, seg_off.data(), seg_off.size());
+    if (!rc) rc = upload(m->win_nbr, nbr.data(), nbr.size());
+    if (!rc) rc = upload(m->win_alias, alias.data(), alias.size());
+    if (!rc) rc = upload(m->win_csign, csign.data(), csign.size());
+    w.ent = m->win_ent; w.desc = m->win_desc; w.seg = m->win_seg; w.seg_off = m->win_seg_off;
+    w.nbr = m->win_nbr; w.alias = m->win_alias;
+    w.csign = m->win_csign;
+    if (!rc) rc = upload(m->win, &w, 1);
+    m->win_host = w;
+    return rc;
+}
+
 extern "C" {
 
 int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
@@ -2215,6 +2367,7 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                 }
             }
             if (!rc && bin && m->brows && m->fix_shift > 0) rc = build_local_field_tables(m, t, sb);
+            if (!rc && bin) rc = build_window_tables(m, t, sb);
             m->binary = !rc;
         }
     }
