@@ -224,7 +224,8 @@ struct LayerW {            // weights of one layer as seen by the kernel (shared
     const float *W, *b, *G, *gb;
 };
 
-// Evaluate one layer for the sites list[pos0 .. pos0+cnt) (or direct0 + 0..cnt-1).  Inputs come from level lvl
+// Evaluate one layer for the sites list[pos0 .. pos0+cnt), or (direct0) the rows *direct0 + 0..cnt-1 of all replicas'
+// caches, row r N + s being site s of replica r.  Inputs come from level lvl
 // (cache patched with the step's values, or unpatched when slot == nullptr).  For every site and group of 4
 // consecutive output columns, `sink(pos, col0, v[4])` receives the activated outputs (pos < 0: padding lane).
 template <typename Sink>
@@ -294,8 +295,10 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
         //    thread with their slot-map loads in flight together.
         for (int mm = tid; mm < tm; mm += nt) {
             const int64_t s = direct0 ? (*direct0 + pos0 + t0 + mm) : list[pos0 + t0 + mm];
-            int32_t b, k[3]; coords(m, s, b, k);
+            const int32_t rr = direct0 ? (int32_t)(s / m.N) : 0;
+            int32_t b, k[3]; coords(m, s - (int64_t)rr * m.N, b, k);
             tsite[mm] = (int32_t)s;
+            if (direct0) tslot[mm] = rr;                     // the row's replica
             tinv[mm] = m.Sh_inv[b * P];
             tk[mm] = make_int4(b, k[0], k[1], k[2]);
         }
@@ -317,6 +320,7 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
                         const int32_t k[3] = {c.y, c.z, c.w};
                         const int e0 = c.x * P * W + (iq - 1);
                         site[u] = m.Sh_m[e0] ? site_at(m, k, m.Sh_uo + 3 * e0, m.Sh_b[e0]) : -1;
+                        if (direct0 && site[u] >= 0) site[u] += (int64_t)tslot[im] * m.N;
                     }
                 }
                 iq += dq; im += dm;
@@ -329,7 +333,7 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
             for (int u = 0; u < 4; ++u) {
                 const int idx = base + u * nt;
                 if (idx >= tm * PW) continue;
-                if (qu[u] == 0) tslot[mmu[u]] = pv[u];
+                if (qu[u] == 0 && !direct0) tslot[mmu[u]] = pv[u];
                 srcp[idx] = site[u] < 0 ? m.zrow
                           : (pv[u] >= 0 && pv[u] < nlev) ? newl + (size_t)pv[u] * Cin : cache + (size_t)site[u] * Cin;
             }
@@ -1431,36 +1435,37 @@ __global__ void nce_h0_kernel(NceDev m, const int8_t *sigma, int32_t R, float *h
     }
 }
 
-// one layer on all sites: out = layer(in); e accumulation on the last layer (weights read from global memory)
-__global__ void __launch_bounds__(256, 1) nce_layer_all_kernel(NceJob jb, int lvl, int32_t r, const float *in, float *out,
-                                                             float *e_out, int64_t chunk0, int64_t chunk_n) {
+// one layer on all sites of all replicas (`rows` rows of the caches from jb.h0, in, out, e_out): out = layer(in), or the site energies
+// of the last layer.  One launch takes every replica's tiles, a CTA tiles blockIdx.x, blockIdx.x + gridDim.x, ...: a
+// launch per replica and layer left most SMs idle on small cells (2,048 sites x 32
+// replicas, float32 width 64, whole cache: 2,340 -> 724 us; 131,072 x 8, split bf16 width 128: 10.4 -> 9.5 ms)
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB) nce_layer_all_kernel(const __grid_constant__ NceJob jb, int lvl, const float *in, float *out,
+                                                                 float *e_out, int64_t rows) {
     extern __shared__ __align__(16) unsigned char smem[];
     const NceDev &m = jb.m;
-    const int TM = tile_tm(m.D, m.tc, m.mma);
     const SmemPlan sp = SmemPlan::make(m, false);
     float *X = reinterpret_cast<float *>(smem + sp.X);
     int32_t *src = reinterpret_cast<int32_t *>(smem + sp.src);
-    const int64_t per = ((chunk_n + gridDim.x - 1) / gridDim.x + TM - 1) / TM * TM;
-    const int64_t a = chunk0 + (int64_t)blockIdx.x * per, cnt = max((int64_t)0, min(per, chunk0 + chunk_n - a));
-    if (cnt <= 0) return;
     __shared__ __align__(8) uint64_t tc_mbar;
     __shared__ uint32_t tc_slot;
     TcCtx tcx;
     if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, &tc_mbar, &tc_slot);
     TcCtx *tcp = m.tc ? &tcx : nullptr;
-    const float *h0 = jb.h0 + (size_t)r * m.N * m.C0;
+    const float *h0 = jb.h0;
+    const int64_t row0 = 0;
     const int D = m.D, ncg = D / 4;
     LayerW LW; LW.W = m.Wc[lvl]; LW.b = m.bias[lvl]; LW.G = m.gate ? m.G[lvl] : nullptr; LW.gb = m.gate ? m.gb[lvl] : nullptr;
     if (out) {
-        layer_tiles(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, cnt, &a, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
-            if (pos >= 0) *reinterpret_cast<float4 *>(out + (size_t)(a + pos) * D + c0) = make_float4(v[0], v[1], v[2], v[3]);
-        }, 0, 1, tcp);
+        layer_tiles(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, rows, &row0, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
+            if (pos >= 0) *reinterpret_cast<float4 *>(out + (size_t)pos * D + c0) = make_float4(v[0], v[1], v[2], v[3]);
+        }, blockIdx.x, gridDim.x, tcp);
     } else {
-        layer_tiles(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, cnt, &a, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
-            const int64_t st = a + pos;
+        layer_tiles(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, rows, &row0, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
+            const int64_t st = pos;
             const float tot = site_energy(v, c0, m.head_w, pos >= 0 ? h0 + (size_t)st * m.C0 : nullptr, m.lin, m.C0, ncg);
             if (pos >= 0 && c0 == 0) e_out[st] = (m.Mb[st % m.nB] > 1) ? tot : 0.f;
-        }, 0, 1, tcp);
+        }, blockIdx.x, gridDim.x, tcp);
     }
     if (m.tc) tc_end(m.D, tcx);
 }
@@ -1985,22 +1990,28 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
     NCE_CUDA(cudaGetLastError());
     NceJob jb = make_nce_job(h, st);
     const size_t xs = tile_smem(m);
-    NCE_CUDA(::nce::raise_smem_limit((const void *)nce_layer_all_kernel, xs));
-    const int blocks = (int)std::min<int64_t>((m.N + tile_tm(m.D, m.tc, m.mma) - 1) / tile_tm(m.D, m.tc, m.mma), 1216);
+    // two CTAs per SM where their tiles fit (the gathers of one hide behind the other's contraction)
+    const bool two = xs <= kStepSmemMax2;
+    auto layer_kern = two ? nce_layer_all_kernel<2> : nce_layer_all_kernel<1>;
+    NCE_CUDA(::nce::raise_smem_limit((const void *)layer_kern, xs));
+    int dev = 0, n_sm = 152;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
     if (m.depth == 0) {
         nce_e0_kernel<<<(int)std::min<int64_t>((tot + 255) / 256, 65535), 256, 0, s>>>(m, st->h0, tot, st->e);
         NCE_CUDA(cudaGetLastError());
     }
-    // hidden layers: hmid[l-1] for l = 1..depth-1, then the last layer into e
-    for (int32_t r = 0; r < st->R && m.depth > 0; ++r) {
-        for (int l = 0; l < m.depth; ++l) {
-            const float *in = l == 0 ? st->h0 + (size_t)r * m.N * m.C0 : st->hmid + ((size_t)(l - 1) * st->R + r) * m.N * m.D;
-            if (l + 1 < m.depth) {
-                float *outp = st->hmid + ((size_t)l * st->R + r) * m.N * m.D;
-                nce_layer_all_kernel<<<blocks, 256, xs, s>>>(jb, l, r, in, outp, nullptr, 0, m.N);
-            } else {
-                nce_layer_all_kernel<<<blocks, 256, xs, s>>>(jb, l, r, in, nullptr, st->e + (size_t)r * m.N, 0, m.N);
-            }
+    // hidden layers: hmid[l-1] for l = 1..depth-1, then the last layer into e; all replicas' rows in one launch each (rows
+    // below 2^31: more replicas take further launches)
+    const int64_t TM = tile_tm(m.D, m.tc, m.mma), rep_per = std::max<int64_t>(1, ((1ll << 31) - 1) / m.N);
+    for (int l = 0; l < m.depth; ++l) {
+        for (int64_t r = 0; r < st->R; r += rep_per) {
+            const int64_t rows = std::min<int64_t>(rep_per, st->R - r) * m.N, tiles = (rows + TM - 1) / TM;
+            jb.h0 = st->h0 + (size_t)r * m.N * m.C0;
+            const float *in = l == 0 ? jb.h0 : st->hmid + ((size_t)(l - 1) * st->R + r) * m.N * m.D;
+            float *outp = l + 1 < m.depth ? st->hmid + ((size_t)l * st->R + r) * m.N * m.D : nullptr;
+            layer_kern<<<(unsigned)std::min<int64_t>(tiles, (int64_t)n_sm * (two ? 2 : 1)), 256, xs, s>>>(
+                jb, l, in, outp, st->e + (size_t)r * m.N, rows);
             NCE_CUDA(cudaGetLastError());
         }
     }
