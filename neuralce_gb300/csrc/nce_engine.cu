@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -37,6 +38,7 @@ int launch_exchange(int32_t R, double *E, double E_scale, const float *beta_slot
                     cudaStream_t s);
 
 constexpr int kMaxLayers = 4;
+constexpr int kTcCols = 64, kTcSlice = 128;   // tcgen05 tiles: output columns staged at a time, K columns of an A slice
 constexpr int kZeroRow = 256;                 // >= every layer's input width
 constexpr double kFix = 1099511627776.0;      // 2^40
 constexpr double kInvFix = 1.0 / 1099511627776.0;
@@ -168,21 +170,23 @@ __host__ __device__ __forceinline__ int x_stride(int kin) { return (kin + 4) & ~
 // for the rest of the kernel, and only drains the abandoned MMAs (bounded) before freeing tensor memory.
 struct TcCtx {
     uint32_t tmem; uint64_t *mbar; uint32_t phase; uint8_t *W; int failed;
+    uint64_t *wbar; uint32_t wphase;          // arrival of a layer's B operand (bulk copy)
 };
 
 // allocation by warp 0 (D columns rounded up to a power of two >= 32) and the mbarrier, for the whole kernel
 __device__ __forceinline__ void tc_begin(int D, TcCtx &tc, uint8_t *wsm, uint64_t *mbar, uint32_t *tslot) {
     if ((threadIdx.x >> 5) == 0) umma::tmem_alloc(tslot, umma::tmem_cols(D));
-    if (threadIdx.x == 0) umma::mbar_init(mbar, 1);
+    if (threadIdx.x == 0) { umma::mbar_init(mbar, 1); umma::mbar_init(mbar + 1, 1); }
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
-    tc.tmem = *tslot; tc.mbar = mbar; tc.phase = 0; tc.W = wsm; tc.failed = 0;
+    tc.tmem = *tslot; tc.mbar = mbar; tc.phase = 0; tc.W = wsm; tc.failed = 0; tc.wbar = mbar + 1; tc.wphase = 0;
 }
 
 __device__ __forceinline__ void tc_end(int D, const TcCtx &tc, uint32_t limit = 1u << 20) {
     // after a wait that gave up, give the abandoned MMAs one more bounded wait before their tensor memory is freed
-    if (tc.failed) umma::mbar_wait(tc.mbar, tc.phase ^ 1u, limit);
+    if (tc.failed == 1) umma::mbar_wait(tc.mbar, tc.phase ^ 1u, limit);
+    if (tc.failed == 2) umma::mbar_wait(tc.wbar, tc.wphase ^ 1u, limit);   // (the same for an abandoned operand copy)
     umma::fence_before();
     __syncthreads();
     if ((threadIdx.x >> 5) == 0) umma::tmem_free(tc.tmem, umma::tmem_cols(D));
@@ -220,6 +224,89 @@ __device__ __forceinline__ void mma_bf16_16816(float d[4], const uint32_t a[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
+// A operand of a tcgen05 tile, rows [0, tm) of the K slice [klo, khi): [h | shell means] in bf16 (hi, and lo when split),
+// core-matrix layout with rows of KS columns.  A thread takes four channels of one site, eight consecutive lanes 32 channels
+// of it: a quarter warp's 16-byte loads then lie in one 128-byte line.  What bounds the gather is the L1's data stage,
+// which takes a wavefront per line a quarter warp touches: lanes spread over eight sites (whose stores fill a core matrix
+// without bank conflicts) cost 26 wavefronts a load and 60 k cycles a width-128 tile, against 27 k this way; four-way
+// conflicts on the one store per twelve loads cost far less.  All partners of a thread are in flight.  Sums run over the partner slots in order, as
+// in the float32 tiles.
+template <int VEC, bool SPLIT>                             // channels a load: 4 (rows of a multiple of 4), 2, 1
+__device__ __forceinline__ void tc_gather(const NceDev &m, const float *const *srcp, const float *tinv, const int4 *tk, int tm, int Cin,
+                                          int klo, int khi, int KS, uint8_t *A0, uint8_t *A1) {
+    const int P = m.P, W = m.W, PW = 1 + P * W;
+    const int nch = (Cin + 3) >> 2;
+    auto load4 = [&](const float *row, int c) -> float4 {
+        if (VEC == 4) return *reinterpret_cast<const float4 *>(row + c);
+        float4 v;
+        if (VEC == 2) {
+            const float2 x = *reinterpret_cast<const float2 *>(row + c);
+            const float2 y = c + 2 < Cin ? *reinterpret_cast<const float2 *>(row + c + 2) : make_float2(0.f, 0.f);
+            v = make_float4(x.x, x.y, y.x, y.y);
+        } else {
+            v.x = row[c]; v.y = c + 1 < Cin ? row[c + 1] : 0.f; v.z = c + 2 < Cin ? row[c + 2] : 0.f; v.w = c + 3 < Cin ? row[c + 3] : 0.f;
+        }
+        return v;
+    };
+    // four channels v into K columns k0 .. (those below k_end and inside the slice) of row r
+    auto store4 = [&](int r, int k0, int k_end, const float4 &v) {
+        uint32_t h0, h1, l0 = 0, l1 = 0;
+        if (SPLIT) { bf16_split(v.x, v.y, h0, l0); bf16_split(v.z, v.w, h1, l1); }
+        else { h0 = bf16x2_bits(__floats2bfloat162_rn(v.x, v.y)); h1 = bf16x2_bits(__floats2bfloat162_rn(v.z, v.w)); }
+        if ((k0 & 3) == 0 && k0 >= klo && k0 + 4 <= min(k_end, khi)) {
+            const uint32_t off = umma::core_off(r, k0 - klo, KS);
+            *reinterpret_cast<uint2 *>(A0 + off) = make_uint2(h0, h1);
+            if (SPLIT) *reinterpret_cast<uint2 *>(A1 + off) = make_uint2(l0, l1);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (k0 + i < klo || k0 + i >= min(k_end, khi)) continue;
+                const uint32_t off = umma::core_off(r, k0 + i - klo, KS);
+                *reinterpret_cast<uint16_t *>(A0 + off) = (uint16_t)((i < 2 ? h0 : h1) >> (16 * (i & 1)));
+                if (SPLIT) *reinterpret_cast<uint16_t *>(A1 + off) = (uint16_t)((i < 2 ? l0 : l1) >> (16 * (i & 1)));
+            }
+        }
+    };
+    // the parts of [self | shell 0 | ...] that the slice meets, one after another: their channels in the slice
+    for (int part = 0; part <= P; ++part) {
+        const int kp = part * Cin, ca = max(klo - kp, 0) >> 2, cb = min((khi - kp + 3) >> 2, nch);   // chunks [ca, cb)
+        const int nc = cb - ca;
+        if (nc <= 0) continue;
+        const int nc8 = nc >> 3;
+        for (int idx = threadIdx.x; idx < ((tm + 3) & ~3) * nc; idx += blockDim.x) {
+            int r, c0;
+            if ((nc & 7) == 0) {                                 // a warp: four sites x eight chunks
+                const int w = idx >> 5, g = w / nc8;
+                r = (g << 2) | ((idx >> 3) & 3); c0 = (((w - g * nc8) << 3) | (idx & 7)) + ca;
+            } else {                                             // consecutive lanes, consecutive chunks of a site
+                r = idx / nc; c0 = idx - r * nc + ca;
+            }
+            c0 <<= 2;
+            if (r >= tm) continue;
+            const float *const *sr = srcp + r * PW;
+            if (part == 0) { store4(r, c0, Cin, load4(sr[0], c0)); continue; }
+            const float *const *pc = sr + 1 + (part - 1) * W;
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (W == 12) {
+                float4 x[12];
+#pragma unroll
+                for (int u = 0; u < 12; ++u) x[u] = load4(pc[u], c0);
+#pragma unroll
+                for (int u = 0; u < 12; ++u) { a.x += x[u].x; a.y += x[u].y; a.z += x[u].z; a.w += x[u].w; }
+            } else {
+#pragma unroll 4
+                for (int u = 0; u < W; ++u) {
+                    const float4 x = load4(pc[u], c0);
+                    a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w;
+                }
+            }
+            const float inv = P == 1 ? tinv[r] : m.Sh_inv[tk[r].x * P + part - 1];
+            a.x *= inv; a.y *= inv; a.z *= inv; a.w *= inv;
+            store4(r, kp + c0, kp + Cin, a);
+        }
+    }
+}
+
 struct LayerW {            // weights of one layer as seen by the kernel (shared or global memory)
     const float *W, *b, *G, *gb;
 };
@@ -227,16 +314,30 @@ struct LayerW {            // weights of one layer as seen by the kernel (shared
 // Evaluate one layer for the sites list[pos0 .. pos0+cnt), or (direct0) the rows *direct0 + 0..cnt-1 of all replicas'
 // caches, row r N + s being site s of replica r.  Inputs come from level lvl
 // (cache patched with the step's values, or unpatched when slot == nullptr).  For every site and group of 4
-// consecutive output columns, `sink(pos, col0, v[4])` receives the activated outputs (pos < 0: padding lane).
-template <typename Sink>
+// consecutive output columns, `sink(pos, col0, v[4])` receives the activated outputs (pos < 0: padding lane); with head
+// weights ehw, tcgen05 tiles sum each site's energy themselves (head terms, then the linear term of the layer-0 row
+// esink.row(pos, site, slot), as site_energy does) and hand it to esink.done(pos, site, energy).
+// sum over the D/4 lanes of one site (consecutive lanes of one warp)
+__device__ __forceinline__ float group_sum(float v, int ncg) {
+    for (int o = ncg >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, ncg);
+    return v;
+}
+
+struct NoSink {
+    __device__ const float *row(int64_t, int32_t, int32_t) const { return nullptr; }
+    __device__ void done(int64_t, int32_t, float) const {}
+};
+
+template <typename Sink, typename ESink = NoSink>
 __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const float *cache, const float *newl, const int32_t *slot,
                             int32_t nlev, const int32_t *list, int64_t pos0, int64_t cnt, const int64_t *direct0, float *X,
-                            int32_t *src, Sink sink, int tile_begin = 0, int tile_stride = 1, TcCtx *tc = nullptr) {
+                            int32_t *src, Sink sink, int tile_begin = 0, int tile_stride = 1, TcCtx *tc = nullptr,
+                            const float *ehw = nullptr, const float *lin = nullptr, ESink esink = ESink{}) {
     const NceDev &m = jb.m;
     const int Cin = lvl == 0 ? m.C0 : m.D, D = m.D, P = m.P, W = m.W;
     const int Kin = (1 + P) * Cin, XS = x_stride(Kin);
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int ncg = D / 4, SG = 256 / ncg, TM = tile_tm(D, tc != nullptr, m.mma), MS = TM / SG;
+    const int ncg = D / 4, SG = (tc ? nt : 256) / ncg, TM = tile_tm(D, tc != nullptr, m.mma), MS = TM / SG;
     const int cg = tid % ncg, sg = tid / ncg;
     const int PW = 1 + P * W;
     // row of each site and shell partner: the step's new value, the cache, or a row of zeros (masked partner)
@@ -250,18 +351,20 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
     // fit shared memory: the split form at width 128 takes its self channels, then its shell means); every slice's
     // MMAs accumulate into the same tensor-memory tile
     const int Kp = kpad16(Kin);
-    const int KS = (tc && Kp > m.tc_ks) ? m.tc_ks : Kp, nks = Kp / KS;
+    const int KS = (tc && Kp > m.tc_ks) ? m.tc_ks : Kp, nks = (Kp + KS - 1) / KS;   // (the last slice may be narrower)
     int klo = 0, khi = Kp;                                   // the slice being gathered (all of K off the tcgen05 path)
     uint8_t *A0 = reinterpret_cast<uint8_t *>(X), *A1 = A0 + (size_t)128 * KS * 2;
     if (tc && tc->failed) return;                            // an earlier completion wait gave up: no more tensor work
+    if ((int64_t)tile_begin * TM >= cnt) return;             // no tile for this CTA
     if (tc) {
         // this layer's B operand into shared memory (read by the tensor cores after the first tile barrier)
-        const size_t n16 = (size_t)Kp * D * 2 * (m.tc_split ? 2 : 1) / 16;
-        const uint4 *g = reinterpret_cast<const uint4 *>(m.Wt[lvl]);
-        uint4 *d = reinterpret_cast<uint4 *>(tc->W);
-        for (size_t i = tid; i < n16; i += nt) d[i] = __ldg(g + i);
+        // (one bulk copy, on its way while the first tile is gathered; every thread's accesses to these bytes ended at
+        // the caller's last barrier)
         umma::fence_async_smem();
+        __syncthreads();
+        if (tid == 0) umma::bulk_load(tc->W, m.Wt[lvl], (uint32_t)(Kp * D * 2 * (m.tc_split ? 2 : 1)), tc->wbar);
     }
+    bool w_ready = false;
     auto xput = [&](int ms, int k, float v) {
         if (tc) {
             if (k < klo || k >= khi) return;
@@ -340,11 +443,25 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
         }
         __syncthreads();
         for (int ks = 0; ks < nks; ++ks) {
-        klo = ks * KS; khi = tc ? klo + KS : Kp;
+        klo = ks * KS; khi = tc ? min(klo + KS, Kp) : Kp;
         // 2) X = [h | masked shell means] of the tile's sites: lanes over channels (coalesced rows); masked
         //    partners read the zero row, so every sum runs over all W slots in order
         const float *zr = m.zrow;
-        if (P == 1 && W <= 12 && Cin <= 64 && (Cin & 1) == 0) {
+        if (tc) {
+            auto gather = [&](auto vec, auto split) {
+                tc_gather<decltype(vec)::value, decltype(split)::value>(m, srcp, tinv, tk, tm, Cin, klo, khi, KS, A0, A1);
+            };
+            using V4 = std::integral_constant<int, 4>; using V2 = std::integral_constant<int, 2>; using V1 = std::integral_constant<int, 1>;
+            if (m.tc_split) {
+                if ((Cin & 3) == 0) gather(V4{}, std::true_type{});
+                else if ((Cin & 1) == 0) gather(V2{}, std::true_type{});
+                else gather(V1{}, std::true_type{});
+            } else {
+                if ((Cin & 3) == 0) gather(V4{}, std::false_type{});
+                else if ((Cin & 1) == 0) gather(V2{}, std::false_type{});
+                else gather(V1{}, std::false_type{});
+            }
+        } else if (P == 1 && W <= 12 && Cin <= 64 && (Cin & 1) == 0) {
             // one shell of at most 12 partners: two sites per warp with all 2 x 13 rows' loads in flight at once;
             // a lane takes the channel pair (2 lane, 2 lane + 1) as one 8-byte load
             const int lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
@@ -508,42 +625,97 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
             // 3'') tcgen05: one thread issues the slice's MMAs into tensor memory (the B operand's K-steps of this
             // slice, accumulating onto the previous slices); every thread waits for their completion before the
             // next slice overwrites the A tile
+            if (!w_ready) {                                     // the layer's B operand has arrived (bounded)
+                w_ready = umma::mbar_wait(tc->wbar, tc->wphase);
+                tc->wphase ^= 1u;
+                if (__syncthreads_or(!w_ready)) { if (tid == 0) atomicOr(jb.err, 32); tc->failed = 2; return; }
+            }
             if (tid == 0) {
                 const size_t bo = (size_t)klo * 16;             // K-step klo / 16 of the B tile (256 bytes per step)
                 umma::issue_tile_k(tc->tmem, A0, A1, (uint32_t)KS * 16u, tc->W + bo, tc->W + (size_t)Kp * D * 2 + bo,
-                                   (uint32_t)Kp * 16u, D, KS / 16, m.tc_split ? 3 : 1, ks > 0, tc->mbar);
+                                   (uint32_t)Kp * 16u, D, (khi - klo) / 16, m.tc_split ? 3 : 1, ks > 0, tc->mbar);
             }
             if (!tc_wait(*tc, jb.err)) return;                  // operands and accumulator left alone from here on
             umma::fence_after();
         }
         }   // K slices
         if (tc) {
-            // every warp reads its lane quarter (rows 32 (warp % 4) ..) and half of the columns of the accumulator,
-            // adds the bias, activates and stages the rows in Y (over the A operand) for the sink's CUDA-core mapping
-            const int warp = tid >> 5, q = warp & 3, hh = warp >> 2;
-            const int cw = D / 2 >= 16 ? D / 2 : 16;
-            const int YS = D + 4;
+            // every warp reads its lane quarter (rows 32 (warp % 4) ..) and a share of the accumulator's columns, adds the
+            // bias and activates.  Rows go to the sink through Y (over the A operand), kTcCols columns at a time, in the
+            // CUDA-core mapping (a lane four columns of a site); for site energies each group of four columns is folded
+            // into its head term at once, and only these parts are staged.
+            const int warp = tid >> 5, q = warp & 3, hh = warp >> 2, nq = nt >> 7;
+            const int YC = ehw ? D : min(D, kTcCols), cw = YC / nq >= 16 ? YC / nq : 16;
+            const int YS = ehw ? ncg + 1 : YC + 4;
             float *Y = X;
             const int rrow = q * 32 + (tid & 31);
-            for (int c0 = hh * cw; c0 < min(D, (hh + 1) * cw); c0 += 16) {
-                float v[16];
-                umma::tmem_ld16(tc->tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
+            for (int y0 = 0; y0 < D; y0 += YC) {
+                if (y0 > 0) __syncthreads();                    // the previous columns are read
+                for (int c0 = y0 + hh * cw; c0 < min(y0 + YC, y0 + (hh + 1) * cw); c0 += 16) {
+                    float v[16];
+                    umma::tmem_ld16(tc->tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, v);
 #pragma unroll
-                for (int i = 0; i < 16; i += 4) {
-                    float4 o;
-                    o.x = act_fn_tc(m.act, v[i] + LW.b[c0 + i]); o.y = act_fn_tc(m.act, v[i + 1] + LW.b[c0 + i + 1]);
-                    o.z = act_fn_tc(m.act, v[i + 2] + LW.b[c0 + i + 2]); o.w = act_fn_tc(m.act, v[i + 3] + LW.b[c0 + i + 3]);
-                    *reinterpret_cast<float4 *>(Y + (size_t)rrow * YS + c0 + i) = o;
+                    for (int i = 0; i < 16; i += 4) {
+                        const float4 bi = *reinterpret_cast<const float4 *>(LW.b + c0 + i);
+                        float4 o;
+                        o.x = act_fn_tc(m.act, v[i] + bi.x); o.y = act_fn_tc(m.act, v[i + 1] + bi.y);
+                        o.z = act_fn_tc(m.act, v[i + 2] + bi.z); o.w = act_fn_tc(m.act, v[i + 3] + bi.w);
+                        if (ehw) {                               // the head terms of four columns, as site_energy sums them
+                            const float *hq = ehw + c0 + i;
+                            Y[rrow * YS + ((c0 + i) >> 2)] = fmaf(o.w, hq[3], fmaf(o.z, hq[2], fmaf(o.y, hq[1], fmaf(o.x, hq[0], 0.f))));
+                        } else {
+                            *reinterpret_cast<float4 *>(Y + rrow * YS + c0 - y0 + i) = o;
+                        }
+                    }
+                }
+                umma::fence_before();
+                __syncthreads();
+                if (!ehw) {
+                    const int yg = YC / 4, cl = tid % yg, s0 = tid / yg, st = nt / yg;
+#pragma unroll 4
+                    for (int mm = s0; mm < 128; mm += st) {
+                        const float4 y = *reinterpret_cast<const float4 *>(Y + mm * YS + cl * 4);
+                        float v[4] = {y.x, y.y, y.z, y.w};
+                        sink(mm < tm ? t0 + mm : -1, y0 + cl * 4, v, tsite[mm < tm ? mm : 0], tslot[mm < tm ? mm : 0]);
+                    }
                 }
             }
-            umma::fence_before();
-            __syncthreads();
-#pragma unroll 8
-            for (int i = 0; i < MS; ++i) {
-                const int mm = sg + i * SG;
-                const float4 y = *reinterpret_cast<const float4 *>(Y + (size_t)mm * YS + cg * 4);
-                float v[4] = {y.x, y.y, y.z, y.w};
-                sink(mm < tm ? t0 + mm : -1, cg * 4, v, tsite[mm < tm ? mm : 0], tslot[mm < tm ? mm : 0]);
+            if (ehw) {
+                // the linear layer-0 term: four sites' rows in flight (at most four channels a lane; wider ones in a loop)
+                constexpr int LC = 4;
+                float lv[LC];
+#pragma unroll
+                for (int j = 0; j < LC; ++j) lv[j] = cg + j * ncg < m.C0 ? lin[cg + j * ncg] : 0.f;
+                for (int i0 = 0; i0 < MS; i0 += 4) {
+                    const float *hr[4];
+                    float x[4][LC];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int mm = sg + min(i0 + i, MS - 1) * SG, mc = mm < tm ? mm : 0;
+                        hr[i] = esink.row(mm < tm ? t0 + mm : -1, tsite[mc], tslot[mc]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+#pragma unroll
+                        for (int j = 0; j < LC; ++j) x[i][j] = cg + j * ncg < m.C0 ? hr[i][cg + j * ncg] : 0.f;
+                    float tot[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int mm = sg + min(i0 + i, MS - 1) * SG;
+                        float part = Y[mm * YS + cg];
+#pragma unroll
+                        for (int j = 0; j < LC; ++j) if (cg + j * ncg < m.C0) part = fmaf(x[i][j], lv[j], part);
+                        for (int c = cg + LC * ncg; c < m.C0; c += ncg) part = fmaf(hr[i][c], lin[c], part);
+                        tot[i] = part;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) tot[i] = group_sum(tot[i], ncg);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int mm = sg + min(i0 + i, MS - 1) * SG;
+                        if (i0 + i < MS && mm < tm && cg == 0) esink.done(t0 + mm, tsite[mm], tot[i]);
+                    }
+                }
             }
             __syncthreads();
             continue;
@@ -686,12 +858,6 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
     }
 }
 
-// sum over the D/4 lanes of one site (consecutive lanes of one warp)
-__device__ __forceinline__ float group_sum(float v, int ncg) {
-    for (int o = ncg >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, ncg);
-    return v;
-}
-
 // energy of a site from its last-layer outputs (this lane's 4 columns at c0) and its layer-0 row hr: every lane of
 // the site's group adds its head terms and its share of the linear layer-0 term (channels c0/4, c0/4 + ncg, ...),
 // then one group sum.  The full caches and the local update both use it, so unchanged inputs give identical bits.
@@ -703,6 +869,11 @@ __device__ __forceinline__ float site_energy(const float *v, int c0, const float
         for (int c = c0 >> 2; c < C0; c += ncg) part = fmaf(hr[c], lin[c], part);
     return group_sum(part, ncg);
 }
+
+template <typename Row, typename Done>
+struct EnergySink {
+    const Row &row; const Done &done;
+};
 
 // One MC step of one replica, run by a cluster of CL CTAs (CL = 1: a single CTA).  The leader (rank 0) draws the
 // proposal, builds the receptive field and the layer-0 change; every level's tiles are spread over the cluster;
@@ -1017,20 +1188,21 @@ __device__ void nce_step(const NceJob &jb, int r, int t, int64_t s_idx, NceCtl &
             // loads of one tile site may run ahead of the stores of the previous one
             const float *__restrict__ e_r = e, *__restrict__ h0_r = h0, *__restrict__ nb0_r = nb0;
             float *__restrict__ en_r = en;
+            // (the tile passes the site and its slot value, read while building the tile)
+            auto row = [&](int64_t pos, int32_t site, int32_t p0) -> const float * {
+                if (pos < 0) return m.zrow;
+                return (p0 >= 0 && p0 < n0) ? nb0_r + (size_t)p0 * m.C0 : h0_r + (size_t)site * m.C0;
+            };
+            auto done = [&](int64_t pos, int32_t site, float tot) {
+                const float ev = m.Mb[site % m.nB] > 1 ? tot : 0.f;
+                en_r[pos] = ev;
+                dloc += (unsigned long long)llrint(((double)ev - (double)e_r[site]) * kFix);
+            };
             layer_tiles(jb, lvl, LWs[lvl], cache, newl, slot, ctl.nl[lvl], list, 0, nout, nullptr, X, src,
                         [&](int64_t pos, int c0, const float *v, int32_t site, int32_t p0) {
-                            // the tile passes the site and its slot value (read while building the tile)
-                            const float *hr = nullptr;
-                            const int64_t st = site;
-                            if (pos >= 0) hr = (p0 >= 0 && p0 < n0) ? nb0_r + (size_t)p0 * m.C0 : h0_r + (size_t)st * m.C0;
-                            const float tot = site_energy(v, c0, hw, hr, lin, m.C0, ncg);
-                            if (pos >= 0 && c0 == 0) {
-                                const bool active = m.Mb[site % m.nB] > 1;
-                                const float ev = active ? tot : 0.f;
-                                en_r[pos] = ev;
-                                dloc += (unsigned long long)llrint(((double)ev - (double)e_r[st]) * kFix);
-                            }
-                        }, rank, CL, tc);
+                            const float tot = site_energy(v, c0, hw, pos >= 0 ? row(pos, site, p0) : nullptr, lin, m.C0, ncg);
+                            if (pos >= 0 && c0 == 0) done(pos, site, tot);
+                        }, rank, CL, tc, tc ? hw : nullptr, lin, EnergySink<decltype(row), decltype(done)>{row, done});
         }
     }
     if (L == 0) {
@@ -1139,7 +1311,7 @@ __host__ __device__ inline size_t weight_floats(int depth, int P, int C0, int D,
 // sharing its bytes with dh | ball-0 entries | weights.  dh (the layer-0 change) lives only between the receptive
 // field's build and the first layer, and the B operand is copied in at the start of each layer, so the two share one
 // region.  with_dh = false: the tile part alone (full-cache kernel).  On the tcgen05 path the X tile holds the bf16
-// A operand(s) [128][tc_ks] or the float32 output rows [128][D + 4], whichever is larger.
+// A operand(s) [128][tc_ks] or float32 output rows [128][min(D, kTcCols) + 4], whichever is larger.
 struct SmemPlan {
     size_t dh, X, src, wt, ent, w, dh_bytes, tile_end, total_w;
     __host__ __device__ static SmemPlan make(const NceDev &m, bool with_dh = true) {
@@ -1152,7 +1324,7 @@ struct SmemPlan {
         p.X = 0;
         size_t xb = sizeof(float) * (size_t)TM * x_stride(Kmax);
         if (m.tc) {
-            const size_t ab = (size_t)128 * m.tc_ks * 2 * (m.tc_split ? 2 : 1), yb = sizeof(float) * 128 * (size_t)(m.D + 4);
+            const size_t ab = (size_t)128 * m.tc_ks * 2 * (m.tc_split ? 2 : 1), yb = sizeof(float) * 128 * (size_t)((m.D < kTcCols ? m.D : kTcCols) + 4);
             xb = ab > yb ? ab : yb;
         }
         p.src = al(p.X + xb);
@@ -1169,8 +1341,8 @@ struct SmemPlan {
 
 // MINB = CTAs resident per SM: 1 (all registers) or 2 (at most 128 registers a thread, twice the warps to hide
 // the latency of the gathers and barriers when two CTAs' shared memory fits an SM)
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) nce_chunk_kernel(const __grid_constant__ NceJob jb, int32_t w_smem) {
+template <int MINB, int NT>
+__global__ void __launch_bounds__(NT, MINB) nce_chunk_kernel(const __grid_constant__ NceJob jb, int32_t w_smem) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ NceCtl ctl;
     const int r = blockIdx.x;
@@ -1186,10 +1358,10 @@ __global__ void __launch_bounds__(256, MINB) nce_chunk_kernel(const __grid_const
     int8_t *ent_sig = reinterpret_cast<int8_t *>(ent_pos + 2 * m.w0max);
     LayerW lw[kMaxLayers]; const float *lin, *hw;
     stage_weights(m, w_smem != 0, wbuf, lw, lin, hw);
-    __shared__ __align__(8) uint64_t tc_mbar;
+    __shared__ __align__(8) uint64_t tc_mbar[2];
     __shared__ uint32_t tc_slot;
     TcCtx tcx;
-    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, &tc_mbar, &tc_slot);
+    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
     const int t = jb.slot_of_rep[r];
     double E = jb.E[r];
     int64_t nacc = 0, nnear = 0;
@@ -1205,8 +1377,8 @@ __global__ void __launch_bounds__(256, MINB) nce_chunk_kernel(const __grid_const
 }
 
 // the same chunk with each replica spread over a thread-block cluster of gridDim.x / R CTAs
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) nce_chunk_cluster_kernel(const __grid_constant__ NceJob jb, int32_t w_smem) {
+template <int MINB, int NT>
+__global__ void __launch_bounds__(NT, MINB) nce_chunk_cluster_kernel(const __grid_constant__ NceJob jb, int32_t w_smem) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ NceCtl ctl;
     cg::cluster_group cluster = cg::this_cluster();
@@ -1224,10 +1396,10 @@ __global__ void __launch_bounds__(256, MINB) nce_chunk_cluster_kernel(const __gr
     int8_t *ent_sig = reinterpret_cast<int8_t *>(ent_pos + 2 * m.w0max);
     LayerW lw[kMaxLayers]; const float *lin, *hw;
     stage_weights(m, w_smem != 0, wbuf, lw, lin, hw);
-    __shared__ __align__(8) uint64_t tc_mbar;
+    __shared__ __align__(8) uint64_t tc_mbar[2];
     __shared__ uint32_t tc_slot;
     TcCtx tcx;
-    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, &tc_mbar, &tc_slot);
+    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
     NceCtx cx; cx.rank = rank; cx.CL = CL; cx.lctl = cluster.map_shared_rank(&ctl, 0);
     cluster.sync();
     const int t = jb.slot_of_rep[r];
@@ -1439,20 +1611,20 @@ __global__ void nce_h0_kernel(NceDev m, const int8_t *sigma, int32_t R, float *h
 // of the last layer.  One launch takes every replica's tiles, a CTA tiles blockIdx.x, blockIdx.x + gridDim.x, ...: a
 // launch per replica and layer left most SMs idle on small cells (2,048 sites x 32
 // replicas, float32 width 64, whole cache: 2,340 -> 724 us; 131,072 x 8, split bf16 width 128: 10.4 -> 9.5 ms)
-template <int MINB>
-__global__ void __launch_bounds__(256, MINB) nce_layer_all_kernel(const __grid_constant__ NceJob jb, int lvl, const float *in, float *out,
-                                                                 float *e_out, int64_t rows) {
+template <int MINB, int NT>
+__global__ void __launch_bounds__(NT, MINB) nce_layer_all_kernel(const __grid_constant__ NceJob jb, int lvl, const float *in, float *out,
+                                                                 float *__restrict__ e_out, int64_t rows) {
     extern __shared__ __align__(16) unsigned char smem[];
     const NceDev &m = jb.m;
     const SmemPlan sp = SmemPlan::make(m, false);
     float *X = reinterpret_cast<float *>(smem + sp.X);
     int32_t *src = reinterpret_cast<int32_t *>(smem + sp.src);
-    __shared__ __align__(8) uint64_t tc_mbar;
+    __shared__ __align__(8) uint64_t tc_mbar[2];
     __shared__ uint32_t tc_slot;
     TcCtx tcx;
-    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, &tc_mbar, &tc_slot);
+    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
     TcCtx *tcp = m.tc ? &tcx : nullptr;
-    const float *h0 = jb.h0;
+    const float *__restrict__ h0 = jb.h0;
     const int64_t row0 = 0;
     const int D = m.D, ncg = D / 4;
     LayerW LW; LW.W = m.Wc[lvl]; LW.b = m.bias[lvl]; LW.G = m.gate ? m.G[lvl] : nullptr; LW.gb = m.gate ? m.gb[lvl] : nullptr;
@@ -1461,11 +1633,12 @@ __global__ void __launch_bounds__(256, MINB) nce_layer_all_kernel(const __grid_c
             if (pos >= 0) *reinterpret_cast<float4 *>(out + (size_t)pos * D + c0) = make_float4(v[0], v[1], v[2], v[3]);
         }, blockIdx.x, gridDim.x, tcp);
     } else {
+        auto row = [&](int64_t pos, int32_t, int32_t) -> const float * { return pos >= 0 ? h0 + (size_t)pos * m.C0 : m.zrow; };
+        auto done = [&](int64_t pos, int32_t, float tot) { e_out[pos] = (m.Mb[pos % m.nB] > 1) ? tot : 0.f; };
         layer_tiles(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, rows, &row0, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
-            const int64_t st = pos;
-            const float tot = site_energy(v, c0, m.head_w, pos >= 0 ? h0 + (size_t)st * m.C0 : nullptr, m.lin, m.C0, ncg);
-            if (pos >= 0 && c0 == 0) e_out[st] = (m.Mb[st % m.nB] > 1) ? tot : 0.f;
-        }, blockIdx.x, gridDim.x, tcp);
+            const float tot = site_energy(v, c0, m.head_w, pos >= 0 ? h0 + (size_t)pos * m.C0 : nullptr, m.lin, m.C0, ncg);
+            if (pos >= 0 && c0 == 0) done(pos, 0, tot);
+        }, blockIdx.x, gridDim.x, tcp, tcp ? m.head_w : nullptr, m.lin, EnergySink<decltype(row), decltype(done)>{row, done});
     }
     if (m.tc) tc_end(m.D, tcx);
 }
@@ -1563,18 +1736,23 @@ static int launch_steps(nce_nce_model *h, const NceJob &jb, int cluster, int cta
     const size_t lim = per_sm == 2 ? kStepSmemMax2 : kStepSmemMax;
     const bool w_smem = step_smem(h->dev, true) <= lim;
     const size_t sm = step_smem(h->dev, w_smem);
+    NCE_CHECK(per_sm == 1 || !h->dev.tc || h->dev.D <= 64, "nce_nce_run_chunk: tensor-core tiles of width 128 do not fit 2 CTAs per SM");
     NCE_CHECK(sm <= lim, "nce_nce_run_chunk: %zu bytes of shared memory per CTA do not fit %d CTAs per SM", sm, per_sm);
     const int CL = cluster > 1 ? cluster : 1;
     NCE_CHECK(CL == 1 || CL == 2 || CL == 4 || CL == 8, "nce_nce_run_chunk: cluster must be 1, 2, 4 or 8");
+    // tensor-core forms with an SM of their own: 512 threads, twice the partner rows in flight per tile (55,296 sites x 16,
+    // width 128 split, 12 steps: 3.39 -> 1.77 ms with the gather and the epilogue of the tiles)
+    const bool wide = h->dev.tc && per_sm == 1;
+    const int nt = wide ? 512 : 256;
     if (CL == 1 || h->dev.depth == 0) {
-        auto kern = per_sm == 2 ? nce_chunk_kernel<2> : nce_chunk_kernel<1>;
+        auto kern = per_sm == 2 ? nce_chunk_kernel<2, 256> : wide ? nce_chunk_kernel<1, 512> : nce_chunk_kernel<1, 256>;
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
-        kern<<<jb.R, 256, sm, stream>>>(jb, w_smem ? 1 : 0);
+        kern<<<jb.R, nt, sm, stream>>>(jb, w_smem ? 1 : 0);
     } else {
-        auto kern = per_sm == 2 ? nce_chunk_cluster_kernel<2> : nce_chunk_cluster_kernel<1>;
+        auto kern = per_sm == 2 ? nce_chunk_cluster_kernel<2, 256> : wide ? nce_chunk_cluster_kernel<1, 512> : nce_chunk_cluster_kernel<1, 256>;
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
         cudaLaunchConfig_t cfg; std::memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3((unsigned)(jb.R * CL)); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = sm;
+        cfg.gridDim = dim3((unsigned)(jb.R * CL)); cfg.blockDim = dim3(nt); cfg.dynamicSmemBytes = sm;
         cfg.stream = stream;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1669,10 +1847,10 @@ namespace nce {
 // tiles, no MMA is issued, so nothing ever arrives; the bounded wait gives up after `limit` polls and the kernel
 // takes the same way out as a layer tile (flag 32 in the model's error word, bounded drain, tensor memory freed).
 __global__ void __launch_bounds__(128) nce_tc_wait_selftest_kernel(int32_t *err, uint32_t limit) {
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t slot;
     TcCtx tc;
-    tc_begin(32, tc, nullptr, &mbar, &slot);
+    tc_begin(32, tc, nullptr, mbar, &slot);
     tc_wait(tc, err, limit);                                // nothing was issued: gives up, sets flag 32 and `failed`
     tc_end(32, tc, limit);
 }
@@ -1775,7 +1953,7 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
     m.mma = d->mma;
     m.tc = (d->mma == 2 || d->mma == 4) && d->depth > 0 ? 1 : 0;
     m.tc_split = d->mma == 4 ? 1 : 0;
-    m.tc_ks = kpad16(tile_kin(d->P, d->C0, d->D));     // the whole K extent of the widest layer in one A tile
+    m.tc_ks = std::min(kpad16(tile_kin(d->P, d->C0, d->D)), kTcSlice);
     m.head_b = (float)d->head_b;
     m.n0max = 2 * n0max; m.nmax = 2 * nLmax; m.w0max = n0max;
     NCE_CHECK(d->Rv_loc, "nce_nce_create: Rv_loc required");
@@ -1933,17 +2111,6 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
         if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int32_t));
         if (e != cudaSuccess) rc = fail(NCE_ERR_CUDA, "nce_nce_create: %s", cudaGetErrorString(e));
     }
-    if (!rc && m.tc && step_smem(m, false) > kStepSmemMax) {
-        // the whole A operand does not fit next to the B operand: stage A in two K slices of every layer whose K
-        // extent divides into them (widths 128 split: self channels, then shell means)
-        const int kp_max = kpad16(tile_kin(m.P, m.C0, m.D)), ks = kp_max / 2;
-        bool ok = kp_max % 32 == 0;
-        for (int l = 0; l < m.depth && ok; ++l) {
-            const int kp = kpad16((1 + m.P) * (l == 0 ? m.C0 : m.D));
-            ok = kp <= ks || kp % ks == 0;
-        }
-        if (ok) m.tc_ks = ks;
-    }
     if (!rc && step_smem(m, false) > kStepSmemMax)
         rc = fail(NCE_ERR_UNSUPPORTED, "nce_nce_create: receptive field%s too large for shared memory (%zu bytes)",
                   m.tc ? " and tensor-core tiles" : "", step_smem(m, false));
@@ -1991,8 +2158,9 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
     NceJob jb = make_nce_job(h, st);
     const size_t xs = tile_smem(m);
     // two CTAs per SM where their tiles fit (the gathers of one hide behind the other's contraction)
-    const bool two = xs <= kStepSmemMax2;
-    auto layer_kern = two ? nce_layer_all_kernel<2> : nce_layer_all_kernel<1>;
+    const bool two = xs <= kStepSmemMax2 && !(m.tc && m.D > 64);
+    const int layer_nt = m.tc && !two ? 512 : 256;
+    auto layer_kern = two ? nce_layer_all_kernel<2, 256> : m.tc ? nce_layer_all_kernel<1, 512> : nce_layer_all_kernel<1, 256>;
     NCE_CUDA(::nce::raise_smem_limit((const void *)layer_kern, xs));
     int dev = 0, n_sm = 152;
     cudaGetDevice(&dev);
@@ -2010,7 +2178,7 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
             jb.h0 = st->h0 + (size_t)r * m.N * m.C0;
             const float *in = l == 0 ? jb.h0 : st->hmid + ((size_t)(l - 1) * st->R + r) * m.N * m.D;
             float *outp = l + 1 < m.depth ? st->hmid + ((size_t)l * st->R + r) * m.N * m.D : nullptr;
-            layer_kern<<<(unsigned)std::min<int64_t>(tiles, (int64_t)n_sm * (two ? 2 : 1)), 256, xs, s>>>(
+            layer_kern<<<(unsigned)std::min<int64_t>(tiles, (int64_t)n_sm * (two ? 2 : 1)), layer_nt, xs, s>>>(
                 jb, l, in, outp, st->e + (size_t)r * m.N, rows);
             NCE_CUDA(cudaGetLastError());
         }
