@@ -1215,62 +1215,153 @@ __global__ void ce_bitplane_kernel(const int8_t *__restrict__ sigma, int32_t R, 
     }
 }
 
-// grid (item blocks x row slices, nB, R): threads over the (k0, k1, 32-anchor word) items of anchor basis
-// blockIdx.y, replica blockIdx.z; a small cell's rows are split into slices over more blocks.  Every lane of a
-// warp walks the same rows (lanes past the last item count nothing).
-__global__ void __launch_bounds__(256) ce_energy_bits_kernel(const uint32_t *__restrict__ planes, int32_t P, int32_t d0, int32_t d1,
-                                                              int32_t d2, int32_t W2, const uint32_t *__restrict__ brows,
-                                                              const int4 *__restrict__ bmem, const int32_t *__restrict__ brow_off,
-                                                              const int32_t *__restrict__ brow_n, int32_t n_cols, int32_t slices,
+// The same planes where a row of k2 fills whole words and species are bytes 0 / 1 on one basis site: a lane packs four
+// sites (a multiply gathers the four low bits), eight lanes a word, and the second copy of a row is the first (the
+// general kernel loads a byte a lane, twice: 67 M sites 226 us).
+__global__ void __launch_bounds__(256) ce_bitplane32_kernel(const uint32_t *__restrict__ sigma, int64_t rows, int32_t d2, int32_t W2,
+                                                            uint32_t flip, uint32_t *__restrict__ planes) {
+    const int lane = threadIdx.x & 31, sub = lane & 7;
+    const int Wn = d2 >> 5;                                  // words of a row
+    const int64_t words = rows * Wn;
+    const int64_t stride = ((int64_t)gridDim.x * blockDim.x) >> 3;
+    for (int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5 << 2; w0 < words; w0 += stride) {
+        const int64_t w = w0 + (lane >> 3);                  // a warp packs four words
+        uint32_t x = w < words ? __ldg(sigma + w * 8 + sub) : 0u;
+        x = ((((x & 0x01010101u) * 0x01020408u) >> 24) & 0xfu) << (4 * sub);
+        x |= __shfl_xor_sync(0xffffffffu, x, 1);
+        x |= __shfl_xor_sync(0xffffffffu, x, 2);
+        x |= __shfl_xor_sync(0xffffffffu, x, 4);
+        x ^= flip;
+        if (w < words && sub < 3) {
+            const int64_t row = w / Wn;
+            const int q = (int)(w - row * Wn);
+            uint32_t *out = planes + row * W2;
+            if (sub < 2) out[q + sub * Wn] = x;
+            else if (q == 0) out[W2 - 1] = 0u;               // the word past the second copy
+        }
+    }
+}
+
+// Column sums of the full energy: grid (item blocks x group slices, nB, R).  A thread takes EW (k0, k1, 32-anchor word) items
+// of anchor basis blockIdx.y, replica blockIdx.z.  It first fetches the shifted plane word of every distinct member
+// offset once into its own shared-memory column (a funnel shift of two plane words; the row address is formed once for
+// the offsets that share it), then forms every cluster instance anchored at the site as the XOR of its members' words,
+// three rows at a time through a full adder and two popcounts.  An instance is anchored at its lowest member, so the
+// members of all rows lie in half of the neighbourhood.  What bounds it is the issue rate: about 6 instructions a row and
+// 32 anchors, with two words a thread so that a row's descriptor serves 64.  (Fetching each member of each row again, the
+// earlier form, spent about 22 instructions a member: 1,048,576 sites x 64, whole call 7.34 ms, now 1.61.)
+constexpr int kEnThreads = 64;
+template <int OTH, int EW>
+__global__ void __launch_bounds__(kEnThreads) ce_energy_bits_kernel(const uint32_t *__restrict__ planes, int32_t P, int32_t d0, int32_t d1,
+                                                              int32_t d2, int32_t W2, const uint4 *__restrict__ words,
+                                                              const int32_t *__restrict__ word_off, const uint32_t *__restrict__ rows,
+                                                              const int32_t *__restrict__ grp_off, const uint32_t *__restrict__ grp_info,
+                                                              int32_t n_cols, int32_t slices, int32_t max_words,
                                                               unsigned long long *__restrict__ cv) {
-    extern __shared__ unsigned long long ccnt[];
-    const int b = blockIdx.y, r = blockIdx.z, lane = threadIdx.x & 31;
+    extern __shared__ __align__(16) unsigned char esm[];
+    uint32_t *wsm = reinterpret_cast<uint32_t *>(esm);                    // [word][thread][EW]; the word past the last is 0
+    unsigned long long *ccnt = reinterpret_cast<unsigned long long *>(esm + sizeof(uint32_t) * EW * kEnThreads * (size_t)(max_words + 1));
+    const int b = blockIdx.y, r = blockIdx.z, tid = threadIdx.x, lane = tid & 31;
     const int slice = (int)(blockIdx.x % (unsigned)slices), iblk = (int)(blockIdx.x / (unsigned)slices);
     const int iblocks = (int)(gridDim.x / (unsigned)slices);
-    for (int c = threadIdx.x; c < n_cols; c += blockDim.x) ccnt[c] = 0ull;
+    for (int c = tid; c < n_cols; c += kEnThreads) ccnt[c] = 0ull;
     __syncthreads();
     const int Wn = (d2 + 31) >> 5;
     const int64_t items = (int64_t)d0 * d1 * Wn;
     const uint32_t *pr = planes + (int64_t)r * P * d0 * d1 * W2;
-    const int nall = brow_n[b];
-    const int q0 = (int)((int64_t)nall * slice / slices), q1 = (int)((int64_t)nall * (slice + 1) / slices);
-    const uint32_t *rows = brows + brow_off[b];
+    const uint4 *wl = words + word_off[b];
+    const int nwd = word_off[b + 1] - word_off[b];
+    const int ga = grp_off[b], gall = grp_off[b + 1] - ga;
+    const int g0 = ga + (int)((int64_t)gall * slice / slices), g1 = ga + (int)((int64_t)gall * (slice + 1) / slices);
     auto flush = [&](int col, int acc) {
         const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)acc);
         if (lane == 0 && sum) atomicAdd(&ccnt[col], (unsigned long long)(long long)sum);
     };
-    for (int64_t base = (int64_t)iblk * blockDim.x; base < items; base += (int64_t)iblocks * blockDim.x) {
-        const int64_t it = base + threadIdx.x;
-        const bool live = it < items;
-        const int64_t itc = live ? it : 0;
-        const int w = (int)(itc % Wn);
-        const int64_t kk = itc / Wn;
-        const int k1 = (int)(kk % d1), k0 = (int)(kk / d1);
-        const int nv = live ? min(32, d2 - 32 * w) : 0;
-        const uint32_t mask = nv >= 32 ? 0xffffffffu : ((1u << nv) - 1u);
+    uint32_t *mine = wsm + tid * EW;
+    constexpr int ST = kEnThreads * EW;                        // shared words between two entries of a thread's column
+#pragma unroll
+    for (int e = 0; e < EW; ++e) mine[nwd * ST + e] = 0u;
+    for (int64_t base = (int64_t)iblk * (kEnThreads * EW); base < items; base += (int64_t)iblocks * (kEnThreads * EW)) {
+        int k0[EW], k1[EW], p2[EW];
+        uint32_t mask[EW];
+        int nv = 0;
+#pragma unroll
+        for (int e = 0; e < EW; ++e) {
+            const int64_t it = base + e * kEnThreads + tid;
+            const int64_t itc = it < items ? it : 0;
+            const int w = (int)(itc % Wn), kk = (int)(itc / Wn);
+            k1[e] = kk % d1; k0[e] = kk / d1; p2[e] = 32 * w;
+            const int v = it < items ? min(32, d2 - 32 * w) : 0;
+            mask[e] = v >= 32 ? 0xffffffffu : ((1u << v) - 1u);
+            nv += v;
+        }
+        const uint32_t *row[EW];
+#pragma unroll 4
+        for (int n = 0; n < nwd; ++n) {
+            const uint4 d = __ldg(wl + n);                     // plane | new row << 31, offset (u0, u1, u2)
+            if (d.x >> 31) {
+#pragma unroll
+                for (int e = 0; e < EW; ++e) {
+                    int a0 = k0[e] + (int)d.y; a0 -= a0 >= d0 ? d0 : 0;
+                    int a1 = k1[e] + (int)d.z; a1 -= a1 >= d1 ? d1 : 0;
+                    row[e] = pr + (((int64_t)(d.x & 0x7fffffffu) * d0 + a0) * d1 + a1) * W2;
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < EW; ++e) {
+                const int pos = p2[e] + (int)d.w;
+                const uint32_t *q = row[e] + (pos >> 5);
+                mine[n * ST + e] = __funnelshift_r(__ldg(q), __ldg(q + 1), (unsigned)(pos & 31)) & mask[e];
+            }
+        }
+        uint32_t own[EW];
+#pragma unroll
+        for (int e = 0; e < EW; ++e) own[e] = mine[e];          // word 0: the anchor itself
         int col = -1, acc = 0;
-        for (int q = q0; q < q1; ++q) {
-            const uint32_t rd = __ldg(rows + q);
-            const int c = (int)(rd & 0xffu), nm = (int)((rd >> 8) & 0xfu), st = (int)(rd >> 12);
+#pragma unroll 2
+        for (int g = g0; g < g1; ++g) {
+            const uint32_t info = __ldg(grp_info + g);           // column | rows << 16
+            const int c = (int)(info & 0xffffu);
             if (c != col) {
                 if (col >= 0) flush(col, acc);
                 col = c; acc = 0;
             }
-            uint32_t par = 0;
-            for (int m = 0; m < nm; ++m) {
-                const int4 e = __ldg(bmem + st + m);           // (plane, uo0, uo1, uo2)
-                int a0 = k0 + e.y; a0 -= a0 >= d0 ? d0 : 0;
-                int a1 = k1 + e.z; a1 -= a1 >= d1 ? d1 : 0;
-                const int pos = 32 * w + e.w;
-                const uint32_t *row = pr + (((int64_t)e.x * d0 + a0) * d1 + a1) * W2 + (pos >> 5);
-                par ^= __funnelshift_r(__ldg(row), __ldg(row + 1), (unsigned)(pos & 31));
+            uint32_t par[3][EW];
+#pragma unroll
+            for (int h = 0; h < 3; ++h) {
+                const uint32_t *rd = rows + ((size_t)g * 3 + h) * (OTH + 1);      // shared-memory word offsets
+                uint32_t off[OTH + 1];
+#pragma unroll
+                for (int k = 0; k < OTH + 1; k += 4) {
+                    const uint4 x = __ldg(reinterpret_cast<const uint4 *>(rd + k));
+                    off[k] = x.x; off[k + 1] = x.y; off[k + 2] = x.z; off[k + 3] = x.w;
+                }
+#pragma unroll
+                for (int e = 0; e < EW; ++e) par[h][e] = own[e];
+#pragma unroll
+                for (int k = 0; k < OTH; ++k) {
+                    const uint32_t *x = mine + off[k];
+                    if (EW == 2) {
+                        const uint2 y = *reinterpret_cast<const uint2 *>(x);
+                        par[h][0] ^= y.x; par[h][EW - 1] ^= y.y;
+                    } else {
+                        par[h][0] ^= x[0];
+                    }
+                }
             }
-            acc += nv - 2 * __popc(par & mask);
+            int odd = 0;
+#pragma unroll
+            for (int e = 0; e < EW; ++e) {
+                const uint32_t s = par[0][e] ^ par[1][e] ^ par[2][e];
+                const uint32_t q = (par[0][e] & par[1][e]) | (par[2][e] & (par[0][e] | par[1][e]));
+                odd += __popc(s) + 2 * __popc(q);
+            }
+            acc += (int)(info >> 16) * nv - 2 * odd;
         }
         if (col >= 0) flush(col, acc);
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < n_cols; c += blockDim.x)
+    for (int c = tid; c < n_cols; c += kEnThreads)
         if (ccnt[c]) atomicAdd(cv + (int64_t)r * n_cols + c, ccnt[c]);
 }
 
@@ -1509,9 +1600,12 @@ struct nce_ce_model {
     int64_t *ecol_fix = nullptr; int32_t fix_shift = 0;   // 2 eci per column x 2^fix_shift (exact dE sums, float64 path)
     int32_t n_cols = 0;
     uint32_t *chunks = nullptr; int32_t *n_chunks = nullptr; int32_t max_chunks = 0;
-    // bit-sliced full energy: rows anchored at a site (col | members << 8 | first member << 12) per anchor basis,
-    // members (plane, uo0, uo1, uo2), the point-function column of each plane
-    uint32_t *brows = nullptr; int4 *bmem = nullptr; int32_t *brow_off = nullptr, *brow_n = nullptr;
+    // bit-sliced full energy, per anchor basis: the distinct member offsets (plane | new row << 31, uo0, uo1, uo2), the rows
+    // in groups of three of one column (bw_oth + 1 word indices each) and each group's column and rows; the
+    // point-function column of each plane
+    uint4 *bwords = nullptr; int32_t *bword_off = nullptr, *bgrp_off = nullptr; uint32_t *brows[2] = {nullptr, nullptr}, *bgrp = nullptr;
+    int32_t bw_max = 0, bw_oth = 3;
+    bool plane32 = false; uint32_t plane_flip = 0;    // planes of one basis site with species 0 / 1 (ce_bitplane32_kernel)
     int32_t *plane_pfc = nullptr; int32_t n_planes = 0;
     double *ecol1 = nullptr;                 // eci of each column (full-energy kernel)
     // local-field kernel: per basis the rows containing each neighbourhood entry, the displacement box, and every
@@ -1544,7 +1638,7 @@ static int upload(T *&dst, const T *src, size_t n) {
 
 static int free_model(nce_ce_model *m) {
     void *ptrs[] = {m->loc, m->pfc, m->eci64, m->eci32, m->rv_len, m->nb_b, m->nb_uo, m->pf64, m->pf32, m->act_b,
-                    m->act_nb, m->grp_cum, m->T_b, m->T_uo, m->T_pfc, m->T_eci64, m->T_eci32, m->err, m->sbits, m->bix, m->rcol, m->ecol2_64, m->ecol2_32, m->ecol_fix, m->chunks, m->n_chunks, m->brows, m->bmem, m->brow_off, m->brow_n, m->plane_pfc, m->ecol1,
+                    m->act_nb, m->grp_cum, m->T_b, m->T_uo, m->T_pfc, m->T_eci64, m->T_eci32, m->err, m->sbits, m->bix, m->rcol, m->ecol2_64, m->ecol2_32, m->ecol_fix, m->chunks, m->n_chunks, m->brows[0], m->brows[1], m->bwords, m->bword_off, m->bgrp_off, m->bgrp, m->plane_pfc, m->ecol1,
                     m->staging_base, m->lf_off, m->lf_idx, m->lf_box, m->frows, m->fmem, m->frow_off, m->frow_n,
                     m->win, m->win_ent, m->win_desc, m->win_seg, m->win_seg_off, m->win_nbr, m->win_alias, m->win_csign};
     for (void *p : ptrs) if (p) cudaFree(p);
@@ -1958,7 +2052,7 @@ static int launch_delta(const CEJob &jb, int mo, int n, const int32_t *rep, cons
 namespace nce {
 int ce_model_dims(nce_ce_handle h, int64_t *N, int32_t *n_cols, int32_t *mo, int32_t *binary) {
     NCE_CHECK(h, "null CE handle");
-    *N = h->N; *n_cols = h->n_cols; *mo = h->mo; *binary = (h->binary && h->brows) ? 1 : 0;
+    *N = h->N; *n_cols = h->n_cols; *mo = h->mo; *binary = (h->binary && h->bgrp) ? 1 : 0;
     return NCE_OK;
 }
 }  // namespace nce
@@ -1968,6 +2062,7 @@ using namespace nce;
 static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t precision, double *E, int64_t *cv_out,
                        cudaStream_t s);
 static int field_init_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int64_t *field, cudaStream_t s);
+static int launch_planes(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t W2, uint32_t *planes, cudaStream_t s);
 
 // Tables of the local-field kernel (see ce_lf_chunk_kernel).  The path is enabled when the cell has no aliasing
 // (every neighbourhood entry of a site is a different site: their k-space displacements, taken as representatives in
@@ -2335,38 +2430,103 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                     for (int q = 0; q < 4; ++q) any = any || (sb[(size_t)c * 4 + q] != 0);
                     if (any) { pmap[c] = (int32_t)ppfc.size(); ppfc.push_back(c); }
                 }
-                std::vector<uint32_t> rows; std::vector<int4> mem; std::vector<int32_t> roff(t->nB), rn(t->nB);
-                for (int b = 0; b < t->nB; ++b) {
-                    roff[b] = (int32_t)rows.size();
+                // every instance once (slot 0), anchored at its lowest member (basis and signed offset) of those that
+                // change sign: (anchor basis, column) -> members beside the anchor
+                typedef std::array<int32_t, 4> Mem;              // plane * nB + basis, uo0, uo1, uo2
+                std::vector<std::vector<std::vector<std::vector<Mem>>>> inst((size_t)t->nB, std::vector<std::vector<std::vector<Mem>>>((size_t)t->n_cols));
+                std::vector<char> has_own((size_t)t->nB, 0);
+                int oth = 0;
+                for (int b = 0; b < t->nB; ++b)
                     for (int q = 0; q < t->Rv_len[b]; ++q) {
                         if (t->Rv_slot[(size_t)b * t->J + q] != 0) continue;
-                        const uint32_t start = (uint32_t)mem.size();
-                        int nm = 0;
+                        std::vector<Mem> mem;
                         for (int k = 0; k < t->mo; ++k) {
                             const size_t e = ((size_t)b * t->J + q) * t->mo + k;
                             const int pl = pmap[t->Rv_pfc[e]];
                             if (pl < 0) continue;                          // constant point function (padded member)
-                            const int loc = t->Rv_loc[e];
-                            const size_t nb = (size_t)b * t->n_nbr + loc;
-                            mem.push_back(make_int4(pl * t->nB + t->nb_b[nb], t->nb_uo[3 * nb], t->nb_uo[3 * nb + 1], t->nb_uo[3 * nb + 2]));
-                            ++nm;
+                            const size_t nb = (size_t)b * t->n_nbr + t->Rv_loc[e];
+                            mem.push_back({pl * t->nB + t->nb_b[nb], t->nb_uo[3 * nb], t->nb_uo[3 * nb + 1], t->nb_uo[3 * nb + 2]});
                         }
-                        if (nm > 15 || start >= (1u << 20)) { bin = false; break; }
-                        rows.push_back((uint32_t)t->Rv_col[(size_t)b * t->J + q] | ((uint32_t)nm << 8) | (start << 12));
+                        int anchor = b;
+                        std::vector<Mem> rel;
+                        if (!mem.empty()) {
+                            auto key = [&](const Mem &x) {
+                                std::array<int64_t, 4> z;
+                                for (int c = 0; c < 3; ++c) z[c] = x[c + 1] > t->d[c] / 2 ? (int64_t)x[c + 1] - t->d[c] : x[c + 1];
+                                z[3] = x[0];
+                                return z;
+                            };
+                            size_t lo = 0;
+                            for (size_t k = 1; k < mem.size(); ++k) if (key(mem[k]) < key(mem[lo])) lo = k;
+                            anchor = mem[lo][0] % t->nB;
+                            for (size_t k = 0; k < mem.size(); ++k) {
+                                Mem x = mem[k];
+                                for (int c = 0; c < 3; ++c) { int64_t v = (int64_t)x[c + 1] - mem[lo][c + 1]; x[c + 1] = (int32_t)(v < 0 ? v + t->d[c] : v); }
+                                if (k == lo) rel.insert(rel.begin(), x); else rel.push_back(x);
+                            }
+                        }
+                        inst[anchor][t->Rv_col[(size_t)b * t->J + q]].push_back(rel);
+                        oth = std::max(oth, (int)rel.size() - 1);
                     }
-                    rn[b] = (int32_t)rows.size() - roff[b];
+                m->bw_oth = oth <= 3 ? 3 : 7;
+                std::vector<uint4> words; std::vector<int32_t> word_off(1, 0), grp_off(1, 0);
+                std::vector<uint32_t> idx, info;                 // (groups, 3, bw_oth + 1) word indices; column | rows << 16
+                for (int b = 0; b < t->nB && bin; ++b) {
+                    std::map<Mem, int> at;                       // the anchor's own words first, the others by row
+                    for (const auto &col : inst[b]) for (const auto &rel : col) if (!rel.empty()) at[rel[0]] = 0;
+                    if (at.size() > 1) bin = false;              // (a basis site carries one point-function column)
+                    std::vector<Mem> order;
+                    for (const auto &kv : at) order.push_back(kv.first);
+                    if (order.empty()) order.push_back({0, 0, 0, 0});
+                    std::map<Mem, int> rest;
+                    for (const auto &col : inst[b]) for (const auto &rel : col) for (const auto &x : rel) if (!at.count(x)) rest[x] = 0;
+                    for (const auto &kv : rest) order.push_back(kv.first);
+                    std::map<Mem, int> ix;
+                    for (size_t k = 0; k < order.size(); ++k) {
+                        const Mem &x = order[k];
+                        const bool fresh = k == 0 || x[0] != order[k - 1][0] || x[1] != order[k - 1][1] || x[2] != order[k - 1][2];
+                        words.push_back(make_uint4((uint32_t)x[0] | (fresh ? 0x80000000u : 0u), (uint32_t)x[1], (uint32_t)x[2], (uint32_t)x[3]));
+                        ix[x] = (int)k;
+                    }
+                    const uint32_t zero = (uint32_t)order.size();
+                    m->bw_max = std::max(m->bw_max, (int32_t)zero);
+                    for (int c = 0; c < t->n_cols; ++c)
+                        for (size_t q = 0; q < inst[b][c].size(); q += 3) {
+                            const size_t nr = std::min<size_t>(3, inst[b][c].size() - q);
+                            info.push_back((uint32_t)c | (uint32_t)nr << 16);
+                            for (size_t h = 0; h < 3; ++h) {
+                                std::vector<uint32_t> w((size_t)m->bw_oth + 1, zero);
+                                // a missing row, or one without sign changes, XORs the anchor away
+                                if (h >= nr || inst[b][c][q + h].empty()) w[0] = 0;
+                                else
+                                    for (size_t k = 1; k < inst[b][c][q + h].size(); ++k) w[k - 1] = (uint32_t)ix[inst[b][c][q + h][k]];
+                                idx.insert(idx.end(), w.begin(), w.end());
+                            }
+                        }
+                    word_off.push_back((int32_t)words.size());
+                    grp_off.push_back((int32_t)info.size());
                 }
+                // a thread's column of words must fit shared memory with one word a thread at least
+                if (m->bw_max > 700) bin = false;
                 if (bin && !ppfc.empty()) {
-                    if (!rc) rc = upload(m->brows, rows.data(), rows.size());
-                    if (!rc) rc = upload(m->bmem, mem.data(), mem.size());
-                    if (!rc) rc = upload(m->brow_off, roff.data(), roff.size());
-                    if (!rc) rc = upload(m->brow_n, rn.data(), rn.size());
+                    std::vector<uint32_t> o1(idx), o2(idx);      // as shared-memory word offsets, one and two words a thread
+                    for (auto &v : o1) v *= kEnThreads;
+                    for (auto &v : o2) v *= 2 * kEnThreads;
+                    if (!rc) rc = upload(m->brows[0], o1.data(), o1.size());
+                    if (!rc) rc = upload(m->brows[1], o2.data(), o2.size());
+                    if (!rc) rc = upload(m->bwords, words.data(), words.size());
+                    if (!rc) rc = upload(m->bword_off, word_off.data(), word_off.size());
+                    if (!rc) rc = upload(m->bgrp_off, grp_off.data(), grp_off.size());
+                    if (!rc) rc = upload(m->bgrp, info.data(), info.size());
+                    m->plane32 = t->nB == 1 && t->max_sp <= 2 && ppfc.size() == 1 && t->d[2] % 32 == 0;
+                    m->plane_flip = sb[(size_t)ppfc[0] * 4] ? 0xffffffffu : 0u;
+                    m->plane32 = m->plane32 && sb[(size_t)ppfc[0] * 4] != sb[(size_t)ppfc[0] * 4 + 1];
                     if (!rc) rc = upload(m->plane_pfc, ppfc.data(), ppfc.size());
                     if (!rc) rc = upload(m->ecol1, colv.data(), colv.size());
                     m->n_planes = (int32_t)ppfc.size();
                 }
             }
-            if (!rc && bin && m->brows && m->fix_shift > 0) rc = build_local_field_tables(m, t, sb);
+            if (!rc && bin && m->bgrp && m->fix_shift > 0) rc = build_local_field_tables(m, t, sb);
             if (!rc && bin) rc = build_window_tables(m, t, sb);
             m->binary = !rc;
         }
@@ -2391,7 +2551,7 @@ int nce_ce_energy(nce_ce_handle h, const int8_t *sigma, int32_t R, int32_t preci
 
 int nce_ce_cluster_counts(nce_ce_handle h, const int8_t *sigma, int32_t R, int64_t *cv, void *stream) {
     NCE_CHECK(h && sigma && cv && R >= 1, "nce_ce_cluster_counts: bad argument");
-    NCE_CHECK(h->binary && h->brows, "nce_ce_cluster_counts: needs point functions in {-1, +1}");
+    NCE_CHECK(h->binary && h->bgrp, "nce_ce_cluster_counts: needs point functions in {-1, +1}");
     std::lock_guard<std::mutex> lk(h->mu);
     cudaStream_t s = (cudaStream_t)stream;
     NCE_CUDA(cudaMemsetAsync(cv, 0, sizeof(int64_t) * (size_t)R * h->n_cols, s));
@@ -2408,11 +2568,27 @@ int nce_ce_energy_from_counts(nce_ce_handle h, const int64_t *cv, int32_t R, dou
 
 }  // extern "C"
 
+// the bit planes of R configurations
+static int launch_planes(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t W2, uint32_t *planes, cudaStream_t s) {
+    const int64_t d0d1 = h->d[0] * h->d[1], d2 = h->d[2];
+    if (h->plane32 && ((uintptr_t)sigma & 3) == 0) {             // (N is a multiple of d2: every row stays aligned)
+        const int64_t rows = (int64_t)R * d0d1, words = rows * (d2 / 32);
+        ce_bitplane32_kernel<<<(int)std::min<int64_t>((words + 31) / 32, 1 << 16), 256, 0, s>>>(
+            reinterpret_cast<const uint32_t *>(sigma), rows, (int32_t)d2, W2, h->plane_flip, planes);
+    } else {
+        const int64_t prow = (int64_t)R * h->n_planes * h->nB * d0d1;
+        ce_bitplane_kernel<<<(int)std::min<int64_t>((prow + 7) / 8, 1 << 20), 256, 0, s>>>(
+            sigma, R, h->N, h->nB, d0d1, (int32_t)d2, W2, h->plane_pfc, h->n_planes, h->sbits, planes);
+    }
+    NCE_CUDA(cudaGetLastError());
+    return NCE_OK;
+}
+
 // full energy of R configurations; cv_out (R, n_cols) additionally receives the cluster-vector sums (sign-parity
 // kernel only, zeroed by the caller); E may be null when only the sums are wanted
 static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t precision, double *E, int64_t *cv_out,
                        cudaStream_t s) {
-    if (h->binary && h->brows) {
+    if (h->binary && h->bgrp) {
         // sign-parity full energy, bit-sliced: planes of the configurations, exact column sums, float64 energy
         NCE_CHECK(R <= 65535, "energy: at most 65535 configurations per call");
         const int64_t d0 = h->d[0], d1 = h->d[1], d2 = h->d[2];
@@ -2428,21 +2604,26 @@ static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t 
             cv = (int64_t *)cvs.p;
             NCE_CUDA(cudaMemsetAsync(cv, 0, sizeof(int64_t) * need_c, s));
         }
-        const int64_t prow = (int64_t)R * P * d0 * d1;
-        const int pb = (int)std::min<int64_t>((prow + 7) / 8, 1 << 20);
-        ce_bitplane_kernel<<<pb, 256, 0, s>>>(sigma, R, h->N, h->nB, d0 * d1, (int32_t)d2, W2, h->plane_pfc, h->n_planes, h->sbits,
-                                              (uint32_t *)planes.p);
-        NCE_CUDA(cudaGetLastError());
+        int rc = launch_planes(h, sigma, R, W2, (uint32_t *)planes.p, s);
+        if (rc) return rc;
         const int64_t items = d0 * d1 * ((d2 + 31) / 32);
-        const int64_t ib = std::min<int64_t>((items + 255) / 256, 8192);
-        // small cells: split the rows so that the launch still covers the SMs (about 4 blocks per SM)
         int nsm = 152;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+        // two words a thread where that still fills the SMs several times over; small cells: one, and the rows split into
+        // slices so that the launch covers the SMs (about 4 blocks per SM; every slice fetches the words again)
+        const bool wide = items * h->nB * R >= 16ll * nsm * kEnThreads * 2 &&
+                          sizeof(uint32_t) * 2 * kEnThreads * (size_t)(h->bw_max + 1) <= 100 * 1024;
+        const int per = kEnThreads * (wide ? 2 : 1);
+        const int64_t ib = std::min<int64_t>((items + per - 1) / per, 8192);
         const int64_t have = ib * h->nB * R;
-        const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(32, (4ll * nsm + have - 1) / have));
-        ce_energy_bits_kernel<<<dim3((unsigned)(ib * slices), h->nB, R), 256, sizeof(unsigned long long) * h->n_cols, s>>>(
-            (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->brows, h->bmem, h->brow_off, h->brow_n, h->n_cols, slices,
-            (unsigned long long *)cv);
+        const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(8, (4ll * nsm + have - 1) / have));
+        const size_t sm = sizeof(uint32_t) * per * (size_t)(h->bw_max + 1) + sizeof(unsigned long long) * h->n_cols;
+        auto kern = h->bw_oth == 3 ? (wide ? ce_energy_bits_kernel<3, 2> : ce_energy_bits_kernel<3, 1>)
+                                   : (wide ? ce_energy_bits_kernel<7, 2> : ce_energy_bits_kernel<7, 1>);
+        NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
+        kern<<<dim3((unsigned)(ib * slices), h->nB, R), kEnThreads, sm, s>>>(
+            (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->bwords, h->bword_off, h->brows[wide ? 1 : 0],
+            h->bgrp_off, h->bgrp, h->n_cols, slices, h->bw_max, (unsigned long long *)cv);
         NCE_CUDA(cudaGetLastError());
         if (E) {
             ce_energy_counts_kernel<<<(R + 127) / 128, 128, 0, s>>>(cv, R, h->n_cols, h->ecol1, h->zerolet, E);
@@ -2688,11 +2869,8 @@ static int field_init_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int6
     const int32_t P = h->n_planes * h->nB;
     StreamScratch planes;
     NCE_CUDA(planes.alloc(sizeof(uint32_t) * (size_t)R * P * d0 * d1 * W2, s));
-    const int64_t prow = (int64_t)R * P * d0 * d1;
-    const int pb = (int)std::min<int64_t>((prow + 7) / 8, 1 << 20);
-    ce_bitplane_kernel<<<pb, 256, 0, s>>>(sigma, R, h->N, h->nB, d0 * d1, (int32_t)d2, W2, h->plane_pfc, h->n_planes, h->sbits,
-                                          (uint32_t *)planes.p);
-    NCE_CUDA(cudaGetLastError());
+    int rc = launch_planes(h, sigma, R, W2, (uint32_t *)planes.p, s);
+    if (rc) return rc;
     const int64_t items = d0 * d1 * ((d2 + 31) / 32);
     ce_field_bits_kernel<<<dim3((unsigned)((items + 127) / 128), h->nB, R), 128, 0, s>>>(
         (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->nB, h->N, h->frows, h->fmem, h->frow_off,
