@@ -18,7 +18,10 @@
 
 #include <climits>
 #include <algorithm>
+#include <array>
+#include <cmath>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -66,10 +69,13 @@ struct NceDev {
     int32_t l0bin; const long long *Rv_wfix; const uint8_t *thsign;
     const int32_t *Rv_desc;                   // (nB, J, mo) l0bin member: loc | valid << 16 | sign bits of species 0..3 << 20
     const long long *col_wfix;                // (K + 1) l0bin: the (shared) 2 w 2^40 of each channel's rows
-    // bit-sliced layer 0 (full caches; l0bin with every member on point function 0): per basis, the reverse rows'
-    // members as (basis, uo0, uo1, uo2) or basis -1, each row's channel, and the channel weight (w, float64)
-    int32_t h0bits; const int4 *h0mem; const double *col_w;
-    int32_t h0_slices; const int2 *h0_slice;  // (nB, S + 1) slice starts (first row, first channel); last = (J, C0)
+    // bit-sliced layer 0 (full caches; l0bin with every member on point function 0), per basis: the distinct member offsets
+    // (basis | new row << 31, uo0, uo1, uo2; the site itself first), the reverse rows in groups of seven of one channel
+    // (shared-memory word offsets of the members beside the site, h0_oth + 1 a row), each channel's groups, and its value for
+    // every count of odd products
+    int32_t h0bits, h0_oth, h0_words, h0_wide; const uint4 *h0w; const int32_t *h0w_off; const uint32_t *h0row;
+    const int32_t *h0grp;                     // (nB, C0 + 1) first group of each channel
+    const float *h0lut; const int32_t *h0lut_off;   // (nB, C0)
     // tcgen05 layer contractions (mma 2: bf16, mma 4: split bf16): per layer the weights as the B operand in bf16
     // core-matrix layout ([D][Kp], Kp = Kin rounded up to 16; hi, then lo when split)
     int32_t tc, tc_split; const uint8_t *Wt[kMaxLayers];
@@ -1497,81 +1503,126 @@ __global__ void nce_plane_kernel(NceDev m, const int8_t *__restrict__ sigma, int
     }
 }
 
-// grid (blocks, nB x S, R): threads over the (k0, k1, 32-site word) items of basis blockIdx.y / S, replica
-// blockIdx.z; slice blockIdx.y % S takes the rows and channels [h0s_row, h0s_ch] .. of the next slice (slices cut
-// the rows of a basis at channel boundaries, so small cells still fill the GPU)
-__global__ void __launch_bounds__(128) nce_h0_bits_kernel(NceDev m, const uint32_t *__restrict__ planes, int32_t W2, float *h0) {
-    const int S = m.h0_slices, b = blockIdx.y / S, sl = blockIdx.y % S, r = blockIdx.z;
-    const int2 lo = m.h0_slice[b * (S + 1) + sl], hi = m.h0_slice[b * (S + 1) + sl + 1];   // (first row, first channel)
-    const int d0 = m.d0, d1 = m.d1, d2 = m.d2;
+// Channels of one slice: those whose first group lies in the slice's share of the basis's groups (channel 0, a constant, in
+// the first slice).
+__host__ __device__ inline int h0_first_channel(const int32_t *grp, int C0, int sl, int S) {
+    if (sl == 0) return 0;
+    const int G = grp[C0];
+    int c = 1;
+    while (c < C0 && (int64_t)grp[c] * S < (int64_t)G * sl) ++c;
+    return c;
+}
+
+// grid (blocks of 32 items, nB x S, R), one warp a block: a thread takes one (k0, k1, 32-site word) item of basis blockIdx.y / S
+// and the channels of slice blockIdx.y % S.  It fetches the shifted plane word of every distinct member offset once into
+// its column of shared memory; a row is then the XOR of its members' words.  Seven rows go through four full adders into
+// three words, and those into a vertical counter of the channel's odd rows per site, whose bits are spread to one count a
+// site and staged as counts; the warp writes them out as values (a table per channel, the float64 rule of the rows
+// rounded once) in whole row segments.  Bound by the issue rate (about 10 instructions a row and 32 sites) and, on large
+// caches, by the stores.  (Fetching every member of every row again and writing single values: whole caches of 131,072 sites x 8 4.68 ms,
+// now 4.16; of 2,048 x 32, 718 us, now 390.)
+template <int OTH, int NQ, typename T>
+__global__ void __launch_bounds__(32) nce_h0_bits_kernel(const __grid_constant__ NceDev m, const uint32_t *__restrict__ planes, int32_t W2,
+                                                         int32_t S, float *__restrict__ h0) {
+    extern __shared__ __align__(16) unsigned char hsm[];
+    constexpr int LB = 8 * (int)sizeof(T), NJ = LB;            // a staged count has LB bits: NJ shifts of 32 / LB sites each
+    constexpr uint32_t LM = LB == 8 ? 0x01010101u : 0x00010001u;
+    constexpr int PITCH = 32 + 4 / (int)sizeof(T);              // items a row of counts, odd in words
+    uint32_t *wsm = reinterpret_cast<uint32_t *>(hsm);           // [word][thread]; the word past the last is 0
+    T *stage = reinterpret_cast<T *>(hsm + sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1));   // [site][channel][item]
+    const int b = blockIdx.y / S, sl = blockIdx.y % S, r = blockIdx.z, lane = threadIdx.x;
+    const int d0 = m.d0, d1 = m.d1, d2 = m.d2, C0 = m.C0;
+    const int32_t *grp = m.h0grp + b * (C0 + 1);
+    const int ca = h0_first_channel(grp, C0, sl, S), cb = sl + 1 == S ? C0 : h0_first_channel(grp, C0, sl + 1, S), nch = cb - ca;
+    if (nch <= 0) return;
     const int Wn = (d2 + 31) >> 5;
     const int64_t items = (int64_t)d0 * d1 * Wn;
-    const int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= items) return;
-    const int w = (int)(it % Wn);
-    const int64_t kk = it / Wn;
-    const int k1 = (int)(kk % d1), k0 = (int)(kk / d1);
-    const int nv = min(32, d2 - 32 * w);
-    const uint32_t mask = nv >= 32 ? 0xffffffffu : ((1u << nv) - 1u);
-    const uint32_t *pr = planes + (int64_t)r * m.nB * d0 * d1 * W2;
-    const int C0 = m.C0;
+    const int64_t it = (int64_t)blockIdx.x * 32 + lane, itc = it < items ? it : 0;
+    const int w = (int)(itc % Wn), kk = (int)(itc / Wn), k1 = kk % d1, k0 = kk / d1;
+    const int nv = it < items ? min(32, d2 - 32 * w) : 0;
     // site j of the word: canonical index ((k0 d1 + k1) d2 + 32 w + j) nB + b
-    float *out0 = h0 + (((int64_t)r * m.N) + ((int64_t)(k0 * d1 + k1) * d2 + 32 * w) * m.nB + b) * C0;
-    const int64_t sstride = (int64_t)m.nB * C0;
-    if (m.Mb[b] < 2) {                                       // inactive sites: zeros
-        for (int j = 0; j < nv; ++j) for (int c = sl ? lo.y : 0; c < hi.y; ++c) out0[j * sstride + c] = 0.f;
-        return;
-    }
-    if (sl == 0) {
-        const float ch0 = (float)((1.0 - (double)m.mu[0]) / (double)m.sd[0]);
-        for (int j = 0; j < nv; ++j) out0[j * sstride] = ch0;
-    }
-    constexpr int NQ = 13;                                    // vertical counter planes: up to 8191 rows per channel
-    uint32_t cnt[NQ];
-    auto flush = [&](int ch, int nrows) {
-        const double wc = m.col_w[ch], base = (double)m.mu[ch] / (double)m.sd[ch];
-        for (int j = 0; j < nv; ++j) {
-            int odd = 0;
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) odd |= (int)((cnt[q] >> j) & 1u) << q;
-            out0[j * sstride + ch] = (float)((double)(nrows - 2 * odd) * wc - base);
+    const int64_t out0 = (((int64_t)r * m.N) + ((int64_t)kk * d2 + 32 * w) * m.nB + b) * C0;
+    const bool active = m.Mb[b] >= 2;                            // inactive sites: zeros
+    if (active) {
+        const uint32_t *pr = planes + (int64_t)r * m.nB * d0 * d1 * W2;
+        const uint4 *wl = m.h0w + m.h0w_off[b];
+        const int nwd = m.h0w_off[b + 1] - m.h0w_off[b];
+        uint32_t *mine = wsm + lane;
+        const uint32_t *row = pr;
+        mine[nwd * 32] = 0u;
+#pragma unroll 4
+        for (int n = 0; n < nwd; ++n) {
+            const uint4 d = __ldg(wl + n);
+            if (d.x >> 31) {
+                int a0 = k0 + (int)d.y; a0 -= a0 >= d0 ? d0 : 0;
+                int a1 = k1 + (int)d.z; a1 -= a1 >= d1 ? d1 : 0;
+                row = pr + (((int64_t)(d.x & 0x7fffffffu) * d0 + a0) * d1 + a1) * W2;
+            }
+            const int pos = 32 * w + (int)d.w;
+            const uint32_t *q = row + (pos >> 5);
+            mine[n * 32] = __funnelshift_r(__ldg(q), __ldg(q + 1), (unsigned)(pos & 31));
         }
-    };
-    int ch_cur = lo.y, nrows = 0;
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) cnt[q] = 0u;
-    const int4 *mem = m.h0mem + (size_t)b * m.J * m.mo;
-    for (int jr = lo.x; jr < hi.x; ++jr) {
-        const int e = b * m.J + jr;
-        if (m.Rv_wfix[e] == 0) continue;
-        const int ch = m.Rv_col[e] + 1;
-        if (ch != ch_cur) {
-            flush(ch_cur, nrows);
+        const uint32_t own = mine[0];
+        for (int ch = max(ca, 1); ch < cb; ++ch) {
+            uint32_t cnt[NQ];
 #pragma unroll
             for (int q = 0; q < NQ; ++q) cnt[q] = 0u;
-            for (int c = ch_cur + 1; c < ch; ++c) flush(c, 0);
-            ch_cur = ch; nrows = 0;
-        }
-        uint32_t par = 0;
-        for (int mm = 0; mm < m.mo; ++mm) {
-            const int4 d = mem[jr * m.mo + mm];                // (member basis or -1, uo0, uo1, uo2)
-            if (d.x < 0) continue;
-            int a0 = k0 + d.y; a0 -= a0 >= d0 ? d0 : 0;
-            int a1 = k1 + d.z; a1 -= a1 >= d1 ? d1 : 0;
-            const int pos = 32 * w + d.w;
-            const uint32_t *row = pr + (((int64_t)d.x * d0 + a0) * d1 + a1) * W2 + (pos >> 5);
-            par ^= __funnelshift_r(__ldg(row), __ldg(row + 1), (unsigned)(pos & 31));
-        }
-        // add the odd-parity bits into the vertical counter (ripple carry)
-        uint32_t carry = par & mask;
+            const int g1 = grp[ch + 1];
+            for (int g = grp[ch]; g < g1; ++g) {
+                const uint32_t *rd = m.h0row + (size_t)g * 7 * (OTH + 1);
+                uint32_t v[7];
 #pragma unroll
-        for (int q = 0; q < NQ; ++q) { const uint32_t t = cnt[q] & carry; cnt[q] ^= carry; carry = t; }
-        ++nrows;
+                for (int h = 0; h < 7; ++h) {
+                    v[h] = own;
+#pragma unroll
+                    for (int k = 0; k < OTH + 1; k += 4) {
+                        const uint4 x = __ldg(reinterpret_cast<const uint4 *>(rd + h * (OTH + 1) + k));
+                        v[h] ^= mine[x.x] ^ mine[x.y] ^ mine[x.z];
+                        if (k + 3 < OTH) v[h] ^= mine[x.w];
+                    }
+                }
+                const uint32_t s0 = v[0] ^ v[1] ^ v[2], q0 = (v[0] & v[1]) | (v[2] & (v[0] | v[1]));
+                const uint32_t s1 = v[3] ^ v[4] ^ v[5], q1 = (v[3] & v[4]) | (v[5] & (v[3] | v[4]));
+                const uint32_t w1 = s0 ^ s1 ^ v[6], q2 = (s0 & s1) | (v[6] & (s0 | s1));
+                const uint32_t w2 = q0 ^ q1 ^ q2, w4 = (q0 & q1) | (q2 & (q0 | q1));
+                uint32_t carry = cnt[0] & w1;
+                cnt[0] ^= w1;
+                uint32_t t = (cnt[1] & w2) | (carry & (cnt[1] | w2));
+                cnt[1] ^= w2 ^ carry; carry = t;
+                t = (cnt[2] & w4) | (carry & (cnt[2] | w4));
+                cnt[2] ^= w4 ^ carry; carry = t;
+#pragma unroll
+                for (int q = 3; q < NQ; ++q) { t = cnt[q] & carry; cnt[q] ^= carry; carry = t; }
+            }
+            // one count a site: sites j, j + LB, ... side by side in a word
+#pragma unroll
+            for (int j = 0; j < NJ; ++j) {
+                uint32_t x = 0;
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) x |= ((cnt[q] >> j) & LM) << q;
+#pragma unroll
+                for (int k = 0; k < 32 / LB; ++k) stage[((j + LB * k) * nch + ch - ca) * PITCH + lane] = (T)(x >> (LB * k));
+            }
+        }
     }
-    if (ch_cur < hi.y) flush(ch_cur, nrows);
-#pragma unroll
-    for (int q = 0; q < NQ; ++q) cnt[q] = 0u;
-    for (int c = ch_cur + 1; c < hi.y; ++c) flush(c, 0);
+    __syncwarp();
+    const float ch0 = (float)((1.0 - (double)m.mu[0]) / (double)m.sd[0]);
+    const int64_t sstride = (int64_t)m.nB * C0;
+    const int32_t *lo = m.h0lut_off + b * C0 + ca;
+    const int dj = 32 / nch, dc = 32 - dj * nch;
+    for (int i = 0; i < 32; ++i) {                               // the items one after another, (site, channel) by lanes
+        const int n = __shfl_sync(0xffffffffu, nv, i);
+        float *out = h0 + __shfl_sync(0xffffffffu, out0, i) + ca;
+        int j = lane / nch, c = lane - j * nch;
+#pragma unroll 4
+        for (; j < n;) {
+            float v = 0.f;
+            if (active) v = ca + c == 0 ? ch0 : __ldg(m.h0lut + __ldg(lo + c) + (int)stage[(j * nch + c) * PITCH + i]);
+            out[j * sstride + c] = v;
+            j += dj; c += dc;
+            if (c >= nch) { c -= nch; ++j; }
+        }
+    }
 }
 
 // Layer 0 of every site for general point functions: every reverse row of each site pulled in float64 (fixed
@@ -1676,6 +1727,7 @@ struct nce_nce_model {
     std::vector<void *> allocs;
     std::mutex mu;
     int32_t *err = nullptr;
+    std::vector<int32_t> h0grp;                 // host copy of dev.h0grp (slices of a launch)
     // scratch for R replicas
     int32_t *slot = nullptr, *list = nullptr; float *newbuf = nullptr, *e_new = nullptr; int64_t stride = 0; int32_t R_alloc = 0;
     nce::NcePending *pend = nullptr;            // (R_alloc) swaps kept by nce_nce_local_delta
@@ -2014,62 +2066,76 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
             chk(dup(h, wf.data(), wf.size(), m.Rv_wfix)); chk(dup(h, ts.data(), ts.size(), m.thsign));
             chk(dup(h, dsc.data(), dsc.size(), m.Rv_desc));
             chk(dup(h, cw.data(), cw.size(), m.col_wfix));
-            // bit-sliced layer 0: every member on point function 0, rows of a basis sorted by channel, at most 8191
-            // rows per channel (13-bit counters), channel weights w
+            // bit-sliced layer 0: every member on point function 0, every row with its own site, at most 8191 rows a channel
             bool hb = m.l0bin != 0 && d->C0 >= 2;
-            std::vector<int4> hm(nr, make_int4(-1, 0, 0, 0));
+            typedef std::array<int32_t, 4> Mem;                 // basis, uo0, uo1, uo2
+            std::vector<uint4> words; std::vector<int32_t> word_off(1, 0), grp, lut_off;
+            std::vector<uint32_t> rows; std::vector<float> lut;
+            int oth = 0, most = 0, widest = 0;
+            std::vector<std::vector<std::vector<std::vector<Mem>>>> by((size_t)d->nB, std::vector<std::vector<std::vector<Mem>>>((size_t)d->C0));
             std::vector<double> cwd((size_t)d->C0, 0.0);
-            for (int b = 0; b < d->nB && hb; ++b) {
-                int last = 0, run = 0;
+            for (int b = 0; b < d->nB && hb; ++b)
                 for (int j = 0; j < d->J && hb; ++j) {
                     const size_t e = (size_t)b * d->J + j;
                     if (wf[e] == 0) continue;
                     const int ch = d->Rv_col[e] + 1;
-                    if (ch < last) hb = false;
-                    run = ch == last ? run + 1 : 1; last = ch;
-                    if (run > 8191) hb = false;
                     cwd[ch] = d->Rv_w[e];
+                    std::vector<Mem> mem; bool own = false;
                     for (int k = 0; k < d->mo; ++k) {
                         const size_t i = e * d->mo + k;
                         if (!d->Rv_m[i]) continue;
                         if (d->Rv_p[i] != 0) hb = false;
-                        hm[i] = make_int4(d->Rv_b[i], d->Rv_uo[3 * i], d->Rv_uo[3 * i + 1], d->Rv_uo[3 * i + 2]);
+                        const Mem x = {d->Rv_b[i], d->Rv_uo[3 * i], d->Rv_uo[3 * i + 1], d->Rv_uo[3 * i + 2]};
+                        if (!own && x == Mem{b, 0, 0, 0}) own = true; else mem.push_back(x);
                     }
+                    hb = hb && own;
+                    oth = std::max(oth, (int)mem.size());
+                    by[b][ch].push_back(mem);
+                    most = std::max(most, (int)by[b][ch].size());
                 }
+            hb = hb && most <= 8191 && oth <= 7;
+            const int OT = oth <= 3 ? 3 : 7;
+            for (int b = 0; b < d->nB && hb; ++b) {
+                std::map<Mem, uint32_t> ix;
+                for (const auto &c : by[b]) for (const auto &r : c) for (const auto &x : r) ix[x] = 0;
+                ix.erase(Mem{b, 0, 0, 0});
+                std::vector<Mem> order(1, Mem{b, 0, 0, 0});
+                for (const auto &kv : ix) order.push_back(kv.first);
+                ix[order[0]] = 0;
+                for (size_t k = 0; k < order.size(); ++k) {
+                    const Mem &x = order[k];
+                    const bool fresh = k == 0 || x[0] != order[k - 1][0] || x[1] != order[k - 1][1] || x[2] != order[k - 1][2];
+                    words.push_back(make_uint4((uint32_t)x[0] | (fresh ? 0x80000000u : 0u), (uint32_t)x[1], (uint32_t)x[2], (uint32_t)x[3]));
+                    ix[x] = (uint32_t)k * 32u;
+                }
+                const uint32_t zero = (uint32_t)order.size() * 32u;
+                widest = std::max(widest, (int)order.size());
+                word_off.push_back((int32_t)words.size());
+                for (int ch = 0; ch < d->C0; ++ch) {
+                    grp.push_back((int32_t)(rows.size() / (7 * (OT + 1))));
+                    const auto &c = by[b][ch];
+                    for (size_t q = 0; q < c.size(); q += 7)
+                        for (size_t k = 0; k < 7; ++k) {
+                            std::vector<uint32_t> w((size_t)OT + 1, zero);
+                            if (q + k >= c.size()) w[0] = 0;     // a missing row XORs the site's own word away
+                            else for (size_t x = 0; x < c[q + k].size(); ++x) w[x] = ix[c[q + k][x]];
+                            rows.insert(rows.end(), w.begin(), w.end());
+                        }
+                    lut_off.push_back((int32_t)lut.size());
+                    const double base = (double)(float)d->mu[ch] / (double)(float)d->sd[ch];
+                    const int n = (int)c.size();
+                    for (int odd = 0; odd <= n; ++odd) lut.push_back((float)std::fma((double)(n - 2 * odd), cwd[ch], -base));
+                }
+                grp.push_back((int32_t)(rows.size() / (7 * (OT + 1))));
             }
+            hb = hb && widest <= 700;
             if (hb) {
-                chk(dup(h, hm.data(), hm.size(), m.h0mem)); chk(dup(h, cwd.data(), cwd.size(), m.col_w));
-                // slices of each basis's rows, cut where the channel changes, about equal in rows
-                const int S = 8;
-                std::vector<int2> sl((size_t)d->nB * (S + 1));
-                for (int b = 0; b < d->nB; ++b) {
-                    std::vector<int> start_row, start_ch;            // candidate cuts: first row of each channel run
-                    int nrows = 0, last = -1;
-                    for (int j = 0; j < d->J; ++j) {
-                        const size_t e = (size_t)b * d->J + j;
-                        if (wf[e] == 0) continue;
-                        const int ch = d->Rv_col[e] + 1;
-                        if (ch != last) { start_row.push_back(j); start_ch.push_back(ch); last = ch; }
-                        ++nrows;
-                    }
-                    int2 *o = &sl[(size_t)b * (S + 1)];
-                    o[0] = make_int2(0, 1);
-                    int k = 1, seen = 0, ci = 0;
-                    for (int j = 0; j < d->J && k < S; ++j) {
-                        const size_t e = (size_t)b * d->J + j;
-                        if (wf[e] == 0) continue;
-                        while (ci < (int)start_row.size() && start_row[ci] < j) ++ci;
-                        if (ci < (int)start_row.size() && start_row[ci] == j && j > 0 && seen >= (int64_t)k * nrows / S &&
-                            start_ch[ci] > o[k - 1].y)
-                            o[k++] = make_int2(j, start_ch[ci]);
-                        ++seen;
-                    }
-                    for (; k <= S; ++k) o[k] = make_int2(d->J, d->C0);      // empty trailing slices
-                    o[S] = make_int2(d->J, d->C0);
-                }
-                chk(dup(h, sl.data(), sl.size(), m.h0_slice));
-                m.h0_slices = S;
+                chk(dup(h, words.data(), words.size(), m.h0w)); chk(dup(h, word_off.data(), word_off.size(), m.h0w_off));
+                chk(dup(h, rows.data(), rows.size(), m.h0row)); chk(dup(h, grp.data(), grp.size(), m.h0grp));
+                chk(dup(h, lut.data(), lut.size(), m.h0lut)); chk(dup(h, lut_off.data(), lut_off.size(), m.h0lut_off));
+                m.h0_oth = OT; m.h0_words = widest; m.h0_wide = most > 255 ? 1 : 0;
                 m.h0bits = 1;
+                h->h0grp = grp;
             }
         }
     }
@@ -2148,9 +2214,27 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
         const int64_t prow = (int64_t)st->R * m.nB * m.d0 * m.d1;
         nce_plane_kernel<<<(int)std::min<int64_t>((prow + 7) / 8, 1 << 20), 256, 0, s>>>(m, st->sigma, st->R, W2, (uint32_t *)planes.p);
         NCE_CUDA(cudaGetLastError());
-        const int64_t items = (int64_t)m.d0 * m.d1 * ((m.d2 + 31) / 32);
-        nce_h0_bits_kernel<<<dim3((unsigned)((items + 127) / 128), m.nB * m.h0_slices, st->R), 128, 0, s>>>(
-            m, (const uint32_t *)planes.p, W2, st->h0);
+        const int64_t items = (int64_t)m.d0 * m.d1 * ((m.d2 + 31) / 32), blocks = (items + 31) / 32;
+        int dv = 0, nsm = 152;
+        cudaGetDevice(&dv);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dv);
+        // channels in slices: enough warps for the SMs (every slice fetches the words again), counts that fit beside the words
+        int S = 1;
+        size_t sm = 0;
+        for (;; S *= 2) {
+            int nch = 0;
+            for (int b = 0; b < m.nB; ++b)
+                for (int sl = 0; sl < S; ++sl) {
+                    const int32_t *g = &h->h0grp[(size_t)b * (m.C0 + 1)];
+                    nch = std::max(nch, (sl + 1 == S ? m.C0 : h0_first_channel(g, m.C0, sl + 1, S)) - h0_first_channel(g, m.C0, sl, S));
+                }
+            sm = sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1) + (size_t)32 * nch * 36 * (m.h0_wide ? 2 : 1);
+            if (S >= 16 || (sm <= 100 * 1024 && blocks * m.nB * st->R * S >= 8ll * nsm)) break;
+        }
+        auto kern = m.h0_wide ? (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 13, uint16_t> : nce_h0_bits_kernel<7, 13, uint16_t>)
+                              : (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 8, uint8_t> : nce_h0_bits_kernel<7, 8, uint8_t>);
+        NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
+        kern<<<dim3((unsigned)blocks, m.nB * S, st->R), 32, sm, s>>>(m, (const uint32_t *)planes.p, W2, S, st->h0);
     } else {
         nce_h0_kernel<<<(int)std::min<int64_t>((tot + 127) / 128, 65535), 128, 0, s>>>(m, st->sigma, st->R, st->h0);
     }
