@@ -1244,12 +1244,11 @@ __global__ void __launch_bounds__(256) ce_bitplane32_kernel(const uint32_t *__re
 
 // Column sums of the full energy: grid (item blocks x group slices, nB, R).  A thread takes EW (k0, k1, 32-anchor word) items
 // of anchor basis blockIdx.y, replica blockIdx.z.  It first fetches the shifted plane word of every distinct member
-// offset once into its own shared-memory column (a funnel shift of two plane words; the row address is formed once for
-// the offsets that share it), then forms every cluster instance anchored at the site as the XOR of its members' words,
+// offset once into its own shared-memory column (a funnel shift of two plane words), then forms every cluster instance anchored at the site as the XOR of its members' words,
 // three rows at a time through a full adder and two popcounts.  An instance is anchored at its lowest member, so the
 // members of all rows lie in half of the neighbourhood.  What bounds it is the issue rate: about 6 instructions a row and
 // 32 anchors, with two words a thread so that a row's descriptor serves 64.  (Fetching each member of each row again, the
-// earlier form, spent about 22 instructions a member: 1,048,576 sites x 64, whole call 7.34 ms, now 1.61.)
+// earlier form, spent about 22 instructions a member: 1,048,576 sites x 64, whole call 7.34 ms, now 1.16.)
 constexpr int kEnThreads = 64;
 template <int OTH, int EW>
 __global__ void __launch_bounds__(kEnThreads) ce_energy_bits_kernel(const uint32_t *__restrict__ planes, int32_t P, int32_t d0, int32_t d1,
@@ -1295,59 +1294,70 @@ __global__ void __launch_bounds__(kEnThreads) ce_energy_bits_kernel(const uint32
             mask[e] = v >= 32 ? 0xffffffffu : ((1u << v) - 1u);
             nv += v;
         }
-        const uint32_t *row[EW];
-#pragma unroll 4
+        // (every word's row address anew: a branch on a shared row would keep the loads of the next words from starting)
+#pragma unroll 8
         for (int n = 0; n < nwd; ++n) {
-            const uint4 d = __ldg(wl + n);                     // plane | new row << 31, offset (u0, u1, u2)
-            if (d.x >> 31) {
-#pragma unroll
-                for (int e = 0; e < EW; ++e) {
-                    int a0 = k0[e] + (int)d.y; a0 -= a0 >= d0 ? d0 : 0;
-                    int a1 = k1[e] + (int)d.z; a1 -= a1 >= d1 ? d1 : 0;
-                    row[e] = pr + (((int64_t)(d.x & 0x7fffffffu) * d0 + a0) * d1 + a1) * W2;
-                }
-            }
+            const uint4 d = __ldg(wl + n);                     // plane, offset (u0, u1, u2)
 #pragma unroll
             for (int e = 0; e < EW; ++e) {
-                const int pos = p2[e] + (int)d.w;
-                const uint32_t *q = row[e] + (pos >> 5);
-                mine[n * ST + e] = __funnelshift_r(__ldg(q), __ldg(q + 1), (unsigned)(pos & 31)) & mask[e];
+                uint32_t a0 = k0[e] + d.y, a1 = k1[e] + d.z;
+                a0 = min(a0, a0 - (uint32_t)d0); a1 = min(a1, a1 - (uint32_t)d1);
+                const uint32_t pos = p2[e] + d.w;
+                const uint32_t *q = pr + (int64_t)((d.x * (uint32_t)d0 + a0) * (uint32_t)d1 + a1) * W2 + (pos >> 5);
+                mine[n * ST + e] = __funnelshift_r(__ldg(q), __ldg(q + 1), pos & 31u) & mask[e];
             }
         }
         uint32_t own[EW];
 #pragma unroll
         for (int e = 0; e < EW; ++e) own[e] = mine[e];          // word 0: the anchor itself
         int col = -1, acc = 0;
-#pragma unroll 2
+        // software pipeline: a group's row descriptors are loaded two groups ahead and its words one group ahead, so that
+        // neither latency stands between two groups (6 to 12 warps an SM are all that the words leave room for)
+        constexpr int NX = 3 * (OTH + 1) / 4;
+        uint4 nx[NX];
+        uint32_t ninfo = 0, winfo = 0, wd[3 * OTH][EW];
+        auto fetch = [&](int g) {
+            const uint4 *rd = reinterpret_cast<const uint4 *>(rows + (size_t)g * 3 * (OTH + 1));
+#pragma unroll
+            for (int k = 0; k < NX; ++k) nx[k] = __ldg(rd + k);
+            ninfo = __ldg(grp_info + g);                         // column | rows << 16
+        };
+        auto load_words = [&]() {
+            uint32_t off[3 * (OTH + 1)];
+#pragma unroll
+            for (int k = 0; k < NX; ++k) { off[4 * k] = nx[k].x; off[4 * k + 1] = nx[k].y; off[4 * k + 2] = nx[k].z; off[4 * k + 3] = nx[k].w; }
+#pragma unroll
+            for (int h = 0; h < 3; ++h)
+#pragma unroll
+                for (int k = 0; k < OTH; ++k) {
+                    const uint32_t *x = mine + off[h * (OTH + 1) + k];
+                    if (EW == 2) {
+                        const uint2 y = *reinterpret_cast<const uint2 *>(x);
+                        wd[h * OTH + k][0] = y.x; wd[h * OTH + k][EW - 1] = y.y;
+                    } else {
+                        wd[h * OTH + k][0] = x[0];
+                    }
+                }
+            winfo = ninfo;
+        };
+        if (g0 < g1) { fetch(g0); load_words(); fetch(min(g0 + 1, g1 - 1)); }
         for (int g = g0; g < g1; ++g) {
-            const uint32_t info = __ldg(grp_info + g);           // column | rows << 16
+            const uint32_t info = winfo;
+            uint32_t par[3][EW];
+#pragma unroll
+            for (int h = 0; h < 3; ++h)
+#pragma unroll
+                for (int e = 0; e < EW; ++e) {
+                    par[h][e] = own[e];
+#pragma unroll
+                    for (int k = 0; k < OTH; ++k) par[h][e] ^= wd[h * OTH + k][e];
+                }
+            load_words();
+            fetch(min(g + 2, g1 - 1));
             const int c = (int)(info & 0xffffu);
             if (c != col) {
                 if (col >= 0) flush(col, acc);
                 col = c; acc = 0;
-            }
-            uint32_t par[3][EW];
-#pragma unroll
-            for (int h = 0; h < 3; ++h) {
-                const uint32_t *rd = rows + ((size_t)g * 3 + h) * (OTH + 1);      // shared-memory word offsets
-                uint32_t off[OTH + 1];
-#pragma unroll
-                for (int k = 0; k < OTH + 1; k += 4) {
-                    const uint4 x = __ldg(reinterpret_cast<const uint4 *>(rd + k));
-                    off[k] = x.x; off[k + 1] = x.y; off[k + 2] = x.z; off[k + 3] = x.w;
-                }
-#pragma unroll
-                for (int e = 0; e < EW; ++e) par[h][e] = own[e];
-#pragma unroll
-                for (int k = 0; k < OTH; ++k) {
-                    const uint32_t *x = mine + off[k];
-                    if (EW == 2) {
-                        const uint2 y = *reinterpret_cast<const uint2 *>(x);
-                        par[h][0] ^= y.x; par[h][EW - 1] ^= y.y;
-                    } else {
-                        par[h][0] ^= x[0];
-                    }
-                }
             }
             int odd = 0;
 #pragma unroll
@@ -1600,7 +1610,7 @@ struct nce_ce_model {
     int64_t *ecol_fix = nullptr; int32_t fix_shift = 0;   // 2 eci per column x 2^fix_shift (exact dE sums, float64 path)
     int32_t n_cols = 0;
     uint32_t *chunks = nullptr; int32_t *n_chunks = nullptr; int32_t max_chunks = 0;
-    // bit-sliced full energy, per anchor basis: the distinct member offsets (plane | new row << 31, uo0, uo1, uo2), the rows
+    // bit-sliced full energy, per anchor basis: the distinct member offsets (plane, uo0, uo1, uo2), the rows
     // in groups of three of one column (bw_oth + 1 word indices each) and each group's column and rows; the
     // point-function column of each plane
     uint4 *bwords = nullptr; int32_t *bword_off = nullptr, *bgrp_off = nullptr; uint32_t *brows[2] = {nullptr, nullptr}, *bgrp = nullptr;
@@ -2484,8 +2494,7 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                     std::map<Mem, int> ix;
                     for (size_t k = 0; k < order.size(); ++k) {
                         const Mem &x = order[k];
-                        const bool fresh = k == 0 || x[0] != order[k - 1][0] || x[1] != order[k - 1][1] || x[2] != order[k - 1][2];
-                        words.push_back(make_uint4((uint32_t)x[0] | (fresh ? 0x80000000u : 0u), (uint32_t)x[1], (uint32_t)x[2], (uint32_t)x[3]));
+                        words.push_back(make_uint4((uint32_t)x[0], (uint32_t)x[1], (uint32_t)x[2], (uint32_t)x[3]));
                         ix[x] = (int)k;
                     }
                     const uint32_t zero = (uint32_t)order.size();
@@ -2509,11 +2518,11 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                 // a thread's column of words must fit shared memory with one word a thread at least
                 if (m->bw_max > 700) bin = false;
                 if (bin && !ppfc.empty()) {
-                    std::vector<uint32_t> o1(idx), o2(idx);      // as shared-memory word offsets, one and two words a thread
-                    for (auto &v : o1) v *= kEnThreads;
-                    for (auto &v : o2) v *= 2 * kEnThreads;
-                    if (!rc) rc = upload(m->brows[0], o1.data(), o1.size());
-                    if (!rc) rc = upload(m->brows[1], o2.data(), o2.size());
+                    for (int k = 0; k < 2; ++k) {                // as shared-memory word offsets: one and two words a thread
+                        std::vector<uint32_t> o(idx);
+                        for (auto &v : o) v *= kEnThreads << k;
+                        if (!rc) rc = upload(m->brows[k], o.data(), o.size());
+                    }
                     if (!rc) rc = upload(m->bwords, words.data(), words.size());
                     if (!rc) rc = upload(m->bword_off, word_off.data(), word_off.size());
                     if (!rc) rc = upload(m->bgrp_off, grp_off.data(), grp_off.size());
@@ -2609,20 +2618,21 @@ static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t 
         const int64_t items = d0 * d1 * ((d2 + 31) / 32);
         int nsm = 152;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-        // two words a thread where that still fills the SMs several times over; small cells: one, and the rows split into
-        // slices so that the launch covers the SMs (about 4 blocks per SM; every slice fetches the words again)
-        const bool wide = items * h->nB * R >= 16ll * nsm * kEnThreads * 2 &&
-                          sizeof(uint32_t) * 2 * kEnThreads * (size_t)(h->bw_max + 1) <= 100 * 1024;
-        const int per = kEnThreads * (wide ? 2 : 1);
+        // two words a thread where that still fills the SMs several times over (a row's descriptor and addresses serve both; four
+        // left too few warps: no faster); small cells: one, and the rows split into slices so that the launch covers the SMs
+        // (about 4 blocks per SM; every slice fetches the words again)
+        const int kw = items * h->nB * R >= 16ll * nsm * kEnThreads * 2 &&
+                       sizeof(uint32_t) * 2 * kEnThreads * (size_t)(h->bw_max + 1) <= 100 * 1024;
+        const int per = kEnThreads << kw;
         const int64_t ib = std::min<int64_t>((items + per - 1) / per, 8192);
         const int64_t have = ib * h->nB * R;
         const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(8, (4ll * nsm + have - 1) / have));
         const size_t sm = sizeof(uint32_t) * per * (size_t)(h->bw_max + 1) + sizeof(unsigned long long) * h->n_cols;
-        auto kern = h->bw_oth == 3 ? (wide ? ce_energy_bits_kernel<3, 2> : ce_energy_bits_kernel<3, 1>)
-                                   : (wide ? ce_energy_bits_kernel<7, 2> : ce_energy_bits_kernel<7, 1>);
+        auto kern = h->bw_oth == 3 ? (kw ? ce_energy_bits_kernel<3, 2> : ce_energy_bits_kernel<3, 1>)
+                                   : (kw ? ce_energy_bits_kernel<7, 2> : ce_energy_bits_kernel<7, 1>);
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
         kern<<<dim3((unsigned)(ib * slices), h->nB, R), kEnThreads, sm, s>>>(
-            (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->bwords, h->bword_off, h->brows[wide ? 1 : 0],
+            (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->bwords, h->bword_off, h->brows[kw],
             h->bgrp_off, h->bgrp, h->n_cols, slices, h->bw_max, (unsigned long long *)cv);
         NCE_CUDA(cudaGetLastError());
         if (E) {

@@ -70,12 +70,12 @@ struct NceDev {
     const int32_t *Rv_desc;                   // (nB, J, mo) l0bin member: loc | valid << 16 | sign bits of species 0..3 << 20
     const long long *col_wfix;                // (K + 1) l0bin: the (shared) 2 w 2^40 of each channel's rows
     // bit-sliced layer 0 (full caches; l0bin with every member on point function 0), per basis: the distinct member offsets
-    // (basis | new row << 31, uo0, uo1, uo2; the site itself first), the reverse rows in groups of seven of one channel
+    // (basis, uo0, uo1, uo2; the site itself first), the reverse rows in groups of seven of one channel
     // (shared-memory word offsets of the members beside the site, h0_oth + 1 a row), each channel's groups, and its value for
     // every count of odd products
     int32_t h0bits, h0_oth, h0_words, h0_wide; const uint4 *h0w; const int32_t *h0w_off; const uint32_t *h0row;
     const int32_t *h0grp;                     // (nB, C0 + 1) first group of each channel
-    const float *h0lut; const int32_t *h0lut_off;   // (nB, C0)
+    const float *h0lut; const int32_t *h0lut_off;   // (nB, C0 + 1)
     // tcgen05 layer contractions (mma 2: bf16, mma 4: split bf16): per layer the weights as the B operand in bf16
     // core-matrix layout ([D][Kp], Kp = Kin rounded up to 16; hi, then lo when split)
     int32_t tc, tc_split; const uint8_t *Wt[kMaxLayers];
@@ -1520,16 +1520,17 @@ __host__ __device__ inline int h0_first_channel(const int32_t *grp, int C0, int 
 // site and staged as counts; the warp writes them out as values (a table per channel, the float64 rule of the rows
 // rounded once) in whole row segments.  Bound by the issue rate (about 10 instructions a row and 32 sites) and, on large
 // caches, by the stores.  (Fetching every member of every row again and writing single values: whole caches of 131,072 sites x 8 4.68 ms,
-// now 4.16; of 2,048 x 32, 718 us, now 390.)
+// now 4.07; of 2,048 x 32, 718 us, now 373.)
 template <int OTH, int NQ, typename T>
 __global__ void __launch_bounds__(32) nce_h0_bits_kernel(const __grid_constant__ NceDev m, const uint32_t *__restrict__ planes, int32_t W2,
-                                                         int32_t S, float *__restrict__ h0) {
+                                                         int32_t S, int32_t lut_max, float *__restrict__ h0) {
     extern __shared__ __align__(16) unsigned char hsm[];
     constexpr int LB = 8 * (int)sizeof(T), NJ = LB;            // a staged count has LB bits: NJ shifts of 32 / LB sites each
     constexpr uint32_t LM = LB == 8 ? 0x01010101u : 0x00010001u;
     constexpr int PITCH = 32 + 4 / (int)sizeof(T);              // items a row of counts, odd in words
     uint32_t *wsm = reinterpret_cast<uint32_t *>(hsm);           // [word][thread]; the word past the last is 0
-    T *stage = reinterpret_cast<T *>(hsm + sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1));   // [site][channel][item]
+    float *lut = reinterpret_cast<float *>(wsm + 32 * (size_t)(m.h0_words + 1));    // the slice's channels' values by count
+    T *stage = reinterpret_cast<T *>(lut + lut_max);             // [site][channel][item]
     const int b = blockIdx.y / S, sl = blockIdx.y % S, r = blockIdx.z, lane = threadIdx.x;
     const int d0 = m.d0, d1 = m.d1, d2 = m.d2, C0 = m.C0;
     const int32_t *grp = m.h0grp + b * (C0 + 1);
@@ -1543,42 +1544,53 @@ __global__ void __launch_bounds__(32) nce_h0_bits_kernel(const __grid_constant__
     // site j of the word: canonical index ((k0 d1 + k1) d2 + 32 w + j) nB + b
     const int64_t out0 = (((int64_t)r * m.N) + ((int64_t)kk * d2 + 32 * w) * m.nB + b) * C0;
     const bool active = m.Mb[b] >= 2;                            // inactive sites: zeros
+    const int32_t *lo = m.h0lut_off + b * (C0 + 1) + ca;
+    const int l0 = lo[0];
     if (active) {
+        for (int i = lane; i < lo[nch] - l0; i += 32) lut[i] = __ldg(m.h0lut + l0 + i);
         const uint32_t *pr = planes + (int64_t)r * m.nB * d0 * d1 * W2;
         const uint4 *wl = m.h0w + m.h0w_off[b];
         const int nwd = m.h0w_off[b + 1] - m.h0w_off[b];
         uint32_t *mine = wsm + lane;
-        const uint32_t *row = pr;
         mine[nwd * 32] = 0u;
-#pragma unroll 4
+#pragma unroll 8
         for (int n = 0; n < nwd; ++n) {
             const uint4 d = __ldg(wl + n);
-            if (d.x >> 31) {
-                int a0 = k0 + (int)d.y; a0 -= a0 >= d0 ? d0 : 0;
-                int a1 = k1 + (int)d.z; a1 -= a1 >= d1 ? d1 : 0;
-                row = pr + (((int64_t)(d.x & 0x7fffffffu) * d0 + a0) * d1 + a1) * W2;
-            }
-            const int pos = 32 * w + (int)d.w;
-            const uint32_t *q = row + (pos >> 5);
-            mine[n * 32] = __funnelshift_r(__ldg(q), __ldg(q + 1), (unsigned)(pos & 31));
+            uint32_t a0 = k0 + d.y, a1 = k1 + d.z;
+            a0 = min(a0, a0 - (uint32_t)d0); a1 = min(a1, a1 - (uint32_t)d1);
+            const uint32_t pos = 32u * w + d.w;
+            const uint32_t *q = pr + (int64_t)((d.x * (uint32_t)d0 + a0) * (uint32_t)d1 + a1) * W2 + (pos >> 5);
+            mine[n * 32] = __funnelshift_r(__ldg(q), __ldg(q + 1), pos & 31u);
         }
         const uint32_t own = mine[0];
+        // a group's row descriptors are loaded while the previous group is counted
+        constexpr int NX = 7 * (OTH + 1) / 4;
+        uint4 nx[NX];
+        auto fetch = [&](int g) {
+            const uint4 *rd = reinterpret_cast<const uint4 *>(m.h0row + (size_t)g * 7 * (OTH + 1));
+#pragma unroll
+            for (int k = 0; k < NX; ++k) nx[k] = __ldg(rd + k);
+        };
+        int g = grp[max(ca, 1)];
+        const int glast = grp[cb] - 1;
+        if (g <= glast) fetch(g);
         for (int ch = max(ca, 1); ch < cb; ++ch) {
             uint32_t cnt[NQ];
 #pragma unroll
             for (int q = 0; q < NQ; ++q) cnt[q] = 0u;
-            const int g1 = grp[ch + 1];
-            for (int g = grp[ch]; g < g1; ++g) {
-                const uint32_t *rd = m.h0row + (size_t)g * 7 * (OTH + 1);
+            for (const int g1 = grp[ch + 1]; g < g1; ++g) {
                 uint32_t v[7];
+                uint4 x[NX];
+#pragma unroll
+                for (int k = 0; k < NX; ++k) x[k] = nx[k];
+                fetch(min(g + 1, glast));
 #pragma unroll
                 for (int h = 0; h < 7; ++h) {
-                    v[h] = own;
-#pragma unroll
-                    for (int k = 0; k < OTH + 1; k += 4) {
-                        const uint4 x = __ldg(reinterpret_cast<const uint4 *>(rd + h * (OTH + 1) + k));
-                        v[h] ^= mine[x.x] ^ mine[x.y] ^ mine[x.z];
-                        if (k + 3 < OTH) v[h] ^= mine[x.w];
+                    const uint4 y = x[h * (OTH + 1) / 4];
+                    v[h] = own ^ mine[y.x] ^ mine[y.y] ^ mine[y.z];
+                    if (OTH == 7) {
+                        const uint4 z = x[h * (OTH + 1) / 4 + (OTH == 7 ? 1 : 0)];
+                        v[h] ^= mine[y.w] ^ mine[z.x] ^ mine[z.y] ^ mine[z.z];
                     }
                 }
                 const uint32_t s0 = v[0] ^ v[1] ^ v[2], q0 = (v[0] & v[1]) | (v[2] & (v[0] | v[1]));
@@ -1608,7 +1620,6 @@ __global__ void __launch_bounds__(32) nce_h0_bits_kernel(const __grid_constant__
     __syncwarp();
     const float ch0 = (float)((1.0 - (double)m.mu[0]) / (double)m.sd[0]);
     const int64_t sstride = (int64_t)m.nB * C0;
-    const int32_t *lo = m.h0lut_off + b * C0 + ca;
     const int dj = 32 / nch, dc = 32 - dj * nch;
     for (int i = 0; i < 32; ++i) {                               // the items one after another, (site, channel) by lanes
         const int n = __shfl_sync(0xffffffffu, nv, i);
@@ -1617,7 +1628,7 @@ __global__ void __launch_bounds__(32) nce_h0_bits_kernel(const __grid_constant__
 #pragma unroll 4
         for (; j < n;) {
             float v = 0.f;
-            if (active) v = ca + c == 0 ? ch0 : __ldg(m.h0lut + __ldg(lo + c) + (int)stage[(j * nch + c) * PITCH + i]);
+            if (active) v = ca + c == 0 ? ch0 : lut[__ldg(lo + c) - l0 + (int)stage[(j * nch + c) * PITCH + i]];
             out[j * sstride + c] = v;
             j += dj; c += dc;
             if (c >= nch) { c -= nch; ++j; }
@@ -1727,7 +1738,7 @@ struct nce_nce_model {
     std::vector<void *> allocs;
     std::mutex mu;
     int32_t *err = nullptr;
-    std::vector<int32_t> h0grp;                 // host copy of dev.h0grp (slices of a launch)
+    std::vector<int32_t> h0grp, h0lut_off;      // host copies of dev.h0grp and dev.h0lut_off (slices of a launch)
     // scratch for R replicas
     int32_t *slot = nullptr, *list = nullptr; float *newbuf = nullptr, *e_new = nullptr; int64_t stride = 0; int32_t R_alloc = 0;
     nce::NcePending *pend = nullptr;            // (R_alloc) swaps kept by nce_nce_local_delta
@@ -2104,8 +2115,7 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
                 ix[order[0]] = 0;
                 for (size_t k = 0; k < order.size(); ++k) {
                     const Mem &x = order[k];
-                    const bool fresh = k == 0 || x[0] != order[k - 1][0] || x[1] != order[k - 1][1] || x[2] != order[k - 1][2];
-                    words.push_back(make_uint4((uint32_t)x[0] | (fresh ? 0x80000000u : 0u), (uint32_t)x[1], (uint32_t)x[2], (uint32_t)x[3]));
+                    words.push_back(make_uint4((uint32_t)x[0], (uint32_t)x[1], (uint32_t)x[2], (uint32_t)x[3]));
                     ix[x] = (uint32_t)k * 32u;
                 }
                 const uint32_t zero = (uint32_t)order.size() * 32u;
@@ -2127,6 +2137,7 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
                     for (int odd = 0; odd <= n; ++odd) lut.push_back((float)std::fma((double)(n - 2 * odd), cwd[ch], -base));
                 }
                 grp.push_back((int32_t)(rows.size() / (7 * (OT + 1))));
+                lut_off.push_back((int32_t)lut.size());
             }
             hb = hb && widest <= 700;
             if (hb) {
@@ -2135,7 +2146,7 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
                 chk(dup(h, lut.data(), lut.size(), m.h0lut)); chk(dup(h, lut_off.data(), lut_off.size(), m.h0lut_off));
                 m.h0_oth = OT; m.h0_words = widest; m.h0_wide = most > 255 ? 1 : 0;
                 m.h0bits = 1;
-                h->h0grp = grp;
+                h->h0grp = grp; h->h0lut_off = lut_off;
             }
         }
     }
@@ -2219,22 +2230,25 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
         cudaGetDevice(&dv);
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dv);
         // channels in slices: enough warps for the SMs (every slice fetches the words again), counts that fit beside the words
-        int S = 1;
+        int S = 1, lut_max = 0;
         size_t sm = 0;
         for (;; S *= 2) {
             int nch = 0;
+            lut_max = 0;
             for (int b = 0; b < m.nB; ++b)
                 for (int sl = 0; sl < S; ++sl) {
-                    const int32_t *g = &h->h0grp[(size_t)b * (m.C0 + 1)];
-                    nch = std::max(nch, (sl + 1 == S ? m.C0 : h0_first_channel(g, m.C0, sl + 1, S)) - h0_first_channel(g, m.C0, sl, S));
+                    const int32_t *g = &h->h0grp[(size_t)b * (m.C0 + 1)], *lo = &h->h0lut_off[(size_t)b * (m.C0 + 1)];
+                    const int ca = h0_first_channel(g, m.C0, sl, S), cb = sl + 1 == S ? m.C0 : h0_first_channel(g, m.C0, sl + 1, S);
+                    nch = std::max(nch, cb - ca);
+                    if (cb > ca) lut_max = std::max(lut_max, (lo[cb] - lo[ca] + 3) & ~3);
                 }
-            sm = sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1) + (size_t)32 * nch * 36 * (m.h0_wide ? 2 : 1);
+            sm = sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1) + sizeof(float) * lut_max + (size_t)32 * nch * 36 * (m.h0_wide ? 2 : 1);
             if (S >= 16 || (sm <= 100 * 1024 && blocks * m.nB * st->R * S >= 8ll * nsm)) break;
         }
         auto kern = m.h0_wide ? (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 13, uint16_t> : nce_h0_bits_kernel<7, 13, uint16_t>)
                               : (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 8, uint8_t> : nce_h0_bits_kernel<7, 8, uint8_t>);
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
-        kern<<<dim3((unsigned)blocks, m.nB * S, st->R), 32, sm, s>>>(m, (const uint32_t *)planes.p, W2, S, st->h0);
+        kern<<<dim3((unsigned)blocks, m.nB * S, st->R), 32, sm, s>>>(m, (const uint32_t *)planes.p, W2, S, lut_max, st->h0);
     } else {
         nce_h0_kernel<<<(int)std::min<int64_t>((tot + 127) / 128, 65535), 128, 0, s>>>(m, st->sigma, st->R, st->h0);
     }
