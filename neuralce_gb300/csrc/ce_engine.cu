@@ -1627,7 +1627,7 @@ struct nce_ce_model {
     // windowed kernel: host copy of the table header (device pointers inside) and its device copy, null when the cell
     // or the cluster set cannot use it
     nce::WinTab win_host; nce::WinTab *win = nullptr;
-    int4 *win_ent = nullptr; uint32_t *win_desc = nullptr; uint2 *win_seg = nullptr; int32_t *win_seg_off = nullptr;
+    int4 *win_ent = nullptr; uint32_t *win_desc = nullptr; uint2 *win_seg = nullptr;
     int16_t *win_nbr = nullptr, *win_alias = nullptr; int32_t *win_csign = nullptr;
 
     int device = 0;
@@ -1650,7 +1650,7 @@ static int free_model(nce_ce_model *m) {
     void *ptrs[] = {m->loc, m->pfc, m->eci64, m->eci32, m->rv_len, m->nb_b, m->nb_uo, m->pf64, m->pf32, m->act_b,
                     m->act_nb, m->grp_cum, m->T_b, m->T_uo, m->T_pfc, m->T_eci64, m->T_eci32, m->err, m->sbits, m->bix, m->rcol, m->ecol2_64, m->ecol2_32, m->ecol_fix, m->chunks, m->n_chunks, m->brows[0], m->brows[1], m->bwords, m->bword_off, m->bgrp_off, m->bgrp, m->plane_pfc, m->ecol1,
                     m->staging_base, m->lf_off, m->lf_idx, m->lf_box, m->frows, m->fmem, m->frow_off, m->frow_n,
-                    m->win, m->win_ent, m->win_desc, m->win_seg, m->win_seg_off, m->win_nbr, m->win_alias, m->win_csign};
+                    m->win, m->win_ent, m->win_desc, m->win_seg, m->win_nbr, m->win_alias, m->win_csign};
     for (void *p : ptrs) if (p) cudaFree(p);
     delete m;
     return NCE_OK;
@@ -1775,7 +1775,11 @@ static int launch_lf(const CEBatch &bt, int mo, int total, int warps, size_t sme
 
 template <typename Acc>
 static int launch_win(const CEBatch &bt, int total, int threads, size_t smem, cudaStream_t s) {
-    auto kern = ce_win_chunk_kernel<Acc>;
+    // as many replicas as SMs or fewer: all the registers of an SM for one CTA
+    int dev = 0, n_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    auto kern = total <= n_sm ? ce_win_chunk_kernel<Acc, 1> : ce_win_chunk_kernel<Acc, 2>;
     NCE_CUDA(::nce::raise_smem_limit((const void *)kern, smem));
     kern<<<total, threads, smem, s>>>(bt);
     NCE_CUDA(cudaGetLastError());
@@ -1873,8 +1877,8 @@ static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *st
     int64_t lf_budget = 0;
     // windowed kernel wherever the sign-parity path runs and every job has its tables (build_window_tables): it was faster
     // at every size and ladder measured, against the step-by-step kernel at its best launch shape (2,048 sites x 32
-    // replicas, 1,000 steps: 1,202 -> 281 us; 131,072 x 256, 300 steps: 1,196 -> 116 us; 256 x 16, 10 steps: 63 -> 26 us;
-    // 24 float32 jobs of 256 to 32,000 sites, 500 steps: 4,154 -> 759 us).  warps and cluster only shape the
+    // replicas, 1,000 steps: 1,202 -> 211 us; 131,072 x 256, 300 steps: 1,196 -> 112 us; 256 x 16, 10 steps: 63 -> 23 us;
+    // 24 float32 jobs of 256 to 32,000 sites, 500 steps: 4,154 -> 722 us).  warps and cluster only shape the
     // step-by-step kernels, which keep the other tables (several basis sites, larger orders, one-cell images).
     bool use_win = use_bin;
     for (int j = 0; j < n_jobs; ++j) use_win = use_win && hs[j]->win != nullptr;
@@ -1882,7 +1886,7 @@ static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *st
     if (use_win) {
         for (int j = 0; j < n_jobs; ++j) {
             const WinTab &w = hs[j]->win_host;
-            smem = std::max(smem, WinLayout::make(w.n_ent, w.n_blk, w.n_seg, hs[j]->n_cols).total);
+            smem = std::max(smem, WinLayout::make(w.n_ent, w.n_blk, hs[j]->n_cols).total);
         }
     } else if (use_lf) {
         size_t t_on = 0, t_off = 0; int64_t maxN = 0;
@@ -2249,39 +2253,39 @@ static int build_window_tables(nce_ce_model *m, const nce_ce_tables *t, const st
     }
     for (const auto &kv : inst) if (kv.second != 0) return NCE_OK;
     // lanes: kWinRows rows of one column each, 32 lanes a block; a column's lanes within a block form one segment
-    std::vector<uint32_t> desc; std::vector<uint2> seg; std::vector<int32_t> seg_off(1, 0);
+    std::vector<uint32_t> desc; std::vector<uint2> seg;
     const uint32_t zero = (uint32_t)n_nbr * 4u, none = zero | (zero << 10) | (zero << 20);
-    int lane = 32;
+    int lane = 32, nseg = 0;                                 // of the block being filled
     for (int c = 0; c < t->n_cols; ++c)
         for (size_t q = 0; q < by_col[c].size(); q += kWinRows) {
-            if (lane == 32) {
-                if (!desc.empty()) seg_off.push_back((int32_t)seg.size());
-                desc.resize(desc.size() + 32 * kWinRows, none); lane = 0;
+            if (lane == 32 || (q == 0 && nseg == kWinSegs)) {
+                desc.resize(desc.size() + 32 * kWinRows, none); seg.resize(seg.size() + kWinSegs, make_uint2(0u, 0u));
+                lane = 0; nseg = 0;
             }
+            if (lane == 0 || q == 0) ++nseg;
+            uint2 &sg = seg[seg.size() - kWinSegs + nseg - 1];
+            sg.x |= 1u << lane; sg.y = 33u * (uint32_t)c;
             uint32_t *d = &desc[desc.size() - 32 * kWinRows];
             for (size_t h = 0; h < kWinRows && q + h < by_col[c].size(); ++h) {
                 uint32_t ix[3] = {zero, zero, zero};
                 for (size_t k = 0; k < by_col[c][q + h].size(); ++k) ix[k] = (uint32_t)by_col[c][q + h][k] * 4u;
                 d[h * 32 + lane] = ix[0] | (ix[1] << 10) | (ix[2] << 20);
             }
-            if ((size_t)seg_off.back() < seg.size() && seg.back().y == (uint32_t)c) seg.back().x |= 1u << lane;
-            else seg.push_back(make_uint2(1u << lane, (uint32_t)c));
             ++lane;
         }
     if (desc.empty()) return NCE_OK;
-    seg_off.push_back((int32_t)seg.size());
-    w.n_blk = (int32_t)seg_off.size() - 1; w.n_seg = (int32_t)seg.size();
-    if (WinLayout::make(w.n_ent, w.n_blk, w.n_seg, t->n_cols).total > 96 * 1024) return NCE_OK;
+    w.n_blk = (int32_t)(seg.size() / kWinSegs);
+    for (int n = 0; n < n_nbr; ++n) w.aliases |= alias[n] >= 0;
+    if (WinLayout::make(w.n_ent, w.n_blk, t->n_cols).total > 96 * 1024) return NCE_OK;
     std::vector<int32_t> csign((size_t)t->n_cols, 2);
     for (int c = 0; c < t->n_cols; ++c) if (sb[(size_t)real * 4] && (order[c] & 1) && order[c] > 0) csign[c] = -2;
     int rc = upload(m->win_ent, ent.data(), ent.size());
     if (!rc) rc = upload(m->win_desc, desc.data(), desc.size());
     if (!rc) rc = upload(m->win_seg, seg.data(), seg.size());
-    if (!rc) rc = upload(m->win_seg_off, seg_off.data(), seg_off.size());
     if (!rc) rc = upload(m->win_nbr, nbr.data(), nbr.size());
     if (!rc) rc = upload(m->win_alias, alias.data(), alias.size());
     if (!rc) rc = upload(m->win_csign, csign.data(), csign.size());
-    w.ent = m->win_ent; w.desc = m->win_desc; w.seg = m->win_seg; w.seg_off = m->win_seg_off;
+    w.ent = m->win_ent; w.desc = m->win_desc; w.seg = m->win_seg;
     w.nbr = m->win_nbr; w.alias = m->win_alias;
     w.csign = m->win_csign;
     if (!rc) rc = upload(m->win, &w, 1);

@@ -23,32 +23,32 @@ constexpr int kWinRows = 7;              // rows a lane: 7 = the most that three
 constexpr int kWinRing = 128;            // proposals in flight (a window reaches 32 steps ahead, drawn 64 ahead)
 constexpr int kWinSwaps = 16;            // swaps evaluated at once: two sites each fill the 32 bits of a word
 constexpr int kWinBatch = 9;             // neighbourhood entries a warp loads at once (141 entries on 16 warps: all)
+constexpr int kWinSegs = 4;               // column segments of a row block
 constexpr int kWinNone = 0x7fffffff;     // "no neighbour": no window index has this value
 
 // per-model tables (device)
 struct WinTab {
     int32_t n_ent;                       // neighbourhood entries, entry 0 the site itself; entry n_ent reads as 0
-    int32_t n_blk, n_seg;                // row blocks of 32 lanes x kWinRows rows; column segments of all blocks
+    int32_t aliases;                     // some displacement has two entries (tiny cells)
+    int32_t n_blk;                       // row blocks of 32 lanes x kWinRows rows
     int32_t lo[3], ext[3];               // offsets per axis lie in [-lo, ext - 1 - lo], ext <= d
     const int4 *ent;                     // (n_ent) offset (u0, u1, u2 in [0, d)) and its window index
     const uint32_t *desc;                // (n_blk, kWinRows, 32) three word indices x 4: bits 2.., 12.., 22..
-    const uint2 *seg;                    // (n_seg) (lanes of the block, column)
-    const int32_t *seg_off;              // (n_blk + 1)
+    const uint2 *seg;                    // (n_blk, kWinSegs) (lanes of the block, 33 x column), lanes 0 when unused
     const int16_t *nbr;                  // entry at each displacement of the window, -1 none
     const int16_t *alias;                // (n_ent) next entry at the same displacement (tiny cells), -1 none
     const int32_t *csign;                // (n_cols) +-2: twice the sign of a column's products for species bits as stored
 };
 
 struct WinLayout {                       // dynamic shared memory
-    size_t words, cnt, desc, seg, seg_off, ent, dcv, nsw, ring, total;
-    __host__ __device__ static WinLayout make(int n_ent, int n_blk, int n_seg, int n_cols) {
+    size_t words, cnt, desc, seg, ent, dcv, nsw, ring, total;
+    __host__ __device__ static WinLayout make(int n_ent, int n_blk, int n_cols) {
         WinLayout L; size_t o = 0;
         auto al = [](size_t x) { return (x + 15) / 16 * 16; };
         L.words = o; o = al(o + 4 * (size_t)(n_ent + 1));
         L.cnt = o; o = al(o + 4 * 33 * (size_t)n_cols);
         L.desc = o; o = al(o + 4 * 32 * (size_t)kWinRows * n_blk);
-        L.seg = o; o = al(o + 8 * (size_t)n_seg);
-        L.seg_off = o; o = al(o + 4 * (size_t)(n_blk + 1));
+        L.seg = o; o = al(o + 8 * (size_t)kWinSegs * n_blk);
         L.ent = o; o = al(o + 16 * (size_t)n_ent);
         L.dcv = o; o = al(o + 4 * (size_t)n_cols);
         L.nsw = o; o = al(o + 2 * (size_t)kWinSwaps * n_cols);
@@ -63,7 +63,8 @@ struct WinCtl {
     uint32_t pred;                       // swaps predicted to be accepted
     int4 site[32];                       // per site: k0, k1, k2, site index
     int32_t del[32];                     // window index of the partner b from site a; kWinNone for b and far pairs
-    int32_t step[kWinSwaps], spa[kWinSwaps];   // step within the window and species of site a, per swap
+    int32_t step[2][kWinSwaps];          // step within the window, per swap (windows in turn)
+    int32_t spa[kWinSwaps];              // species of site a
     long long part[kWinSwaps];           // dE: fixed point or the bits of a float64
     int32_t flags[kWinSwaps];            // 1 accepted, 2 near its threshold
     int32_t nbr[kWinSwaps], same[kWinSwaps];   // first later step whose dE the swap moves; first that shares a site with it
@@ -138,10 +139,13 @@ __device__ __forceinline__ int win_decide_f32(const CEJob &jb, double dE, unsign
     return (logu < -beta * dE ? 1 : 0) | (beta > 0.0 && fabs(dE + logu / beta) < jb.near_eV ? 2 : 0);
 }
 
-// One CTA per replica.  Warp 0 decides and lists windows, the last warp draws proposals while the others count rows; all
-// warps gather the window's words and sum the swaps' dE.  Four barriers a window.
-template <typename Acc>
-__global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_constant__ CEBatch bt) {
+// One CTA per replica.  Warp 0 decides and lists windows while warp 1 keeps the books, the last warp draws proposals while the
+// others count rows; all warps gather the window's words and sum the swaps' dE.  Four barriers a window.  A window takes
+// about 6.9 k cycles on an SM of its own (2,048 sites: words 2.6 k, rows 1.9 k, dE 1.1 k, decision and list 1.4 k), at the hottest
+// replica 20 steps; with one warp keeping everything, 64 registers a thread and uneven column segments it took 10.5 k
+// (1,000 steps of 32 replicas: 281 -> 211 us; 1,048,576 sites x 64, 500 steps: 152 -> 103 us).
+template <typename Acc, int MINB>
+__global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_constant__ CEBatch bt) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr bool FIX = std::is_same<Acc, double>::value;
     __shared__ CEJob sjob;
@@ -157,12 +161,11 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
         reinterpret_cast<int *>(&wt)[i] = reinterpret_cast<const int *>(jb.win)[i];
     __syncthreads();
     const int n_ent = wt.n_ent, n_cols = jb.n_cols, n_blk = wt.n_blk;
-    const WinLayout L = WinLayout::make(n_ent, n_blk, wt.n_seg, n_cols);
+    const WinLayout L = WinLayout::make(n_ent, n_blk, n_cols);
     uint32_t *words = reinterpret_cast<uint32_t *>(smem + L.words);
     int32_t *cnt = reinterpret_cast<int32_t *>(smem + L.cnt);               // [column][site], rows of 33
     uint32_t *desc = reinterpret_cast<uint32_t *>(smem + L.desc);
     uint2 *seg = reinterpret_cast<uint2 *>(smem + L.seg);
-    int32_t *seg_off = reinterpret_cast<int32_t *>(smem + L.seg_off);
     int4 *ent = reinterpret_cast<int4 *>(smem + L.ent);
     int32_t *dcv = reinterpret_cast<int32_t *>(smem + L.dcv);
     int16_t *nsw = reinterpret_cast<int16_t *>(smem + L.nsw);                // [swap][column] of the evaluated swaps
@@ -172,8 +175,7 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
     ring.lnu = reinterpret_cast<float *>(ring.u + kWinRing); ring.del = reinterpret_cast<int32_t *>(ring.lnu + kWinRing);
     int8_t *gsig = jb.sigma + (int64_t)r * jb.N;
     for (int i = tid; i < n_blk * kWinRows * 32; i += nt) desc[i] = __ldg(wt.desc + i);
-    for (int i = tid; i < wt.n_seg; i += nt) seg[i] = __ldg(wt.seg + i);
-    for (int i = tid; i <= n_blk; i += nt) seg_off[i] = __ldg(wt.seg_off + i);
+    for (int i = tid; i < n_blk * kWinSegs; i += nt) seg[i] = __ldg(wt.seg + i);
     for (int i = tid; i < n_ent; i += nt) ent[i] = __ldg(wt.ent + i);
     for (int i = tid; i < 33 * n_cols; i += nt) cnt[i] = 0;
     for (int i = tid; i <= n_ent; i += nt) words[i] = 0;
@@ -190,7 +192,7 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
     const int32_t si = jb.E_samples && jb.sample_interval <= T ? (int32_t)jb.sample_interval : 0;
     int32_t s_next = si;                                     // the next step to sample (1-based)
     const double E0 = jb.E[r];
-    double E = E0, Emin = jb.E_min_rep[r];                  // float32: carried energy and running minimum (warp 0)
+    double E = E0, Emin = jb.E_min_rep[r];                  // float32: carried energy and running minimum (warp 1)
     long long dsum = 0, dmin = 0;                            // float64: the chunk's energy change; this lane's minimum of it
     int32_t nacc = 0, nnear = 0, drawn = 96, s_cur = 0, score = 0;
     for (int q = tid; q < min(96, T); q += nt) win_propose(jb, wt, ring, g0, q, t);
@@ -217,7 +219,8 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
         y = __shfl_xor_sync(0xffffffffu, x, 1); y = __funnelshift_l(y, y, rot1); x = (x & keep1) | (y & ~keep1);
         return x;
     };
-    // warp 0: the window that starts at step s_cur, on the present occupancy
+    int par = 1;                                              // parity of the window in X.step
+    // warp 0: the window that starts at step s_cur, on the present occupancy, into X (X.step of the other parity)
     auto list_window = [&]() {
         const int avail = min(32, T - s_cur);
         const int i = (s_cur + lane) & (kWinRing - 1);
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
         if (in) {
             X.site[2 * rank] = a; X.site[2 * rank + 1] = b;
             X.del[2 * rank] = del; X.del[2 * rank + 1] = kWinNone;
-            X.step[rank] = lane; X.spa[rank] = sa;
+            X.step[par ^ 1][rank] = lane; X.spa[rank] = sa;
         }
         if (lane == 0) { X.s = s_cur; X.n_w = n_w; X.nv = nv; X.pred = pred; }
     };
@@ -250,17 +253,23 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
         const int n_w = X.n_w, nv = X.nv, s_w = X.s;
         const uint32_t pred = X.pred;
         if (n_w == 0) break;
+        par ^= 1;
+        const int32_t *step = X.step[par];
         // what swap v changes, once accepted: the first later swap whose neighbourhood holds one of its sites and the
         // first later step that shares a site with it; apply: flip its two sites in the later swaps' words
         auto touch = [&](int v, const int4 &own, bool apply) {
             const int4 a = X.site[2 * v], b = X.site[2 * v + 1];
-            const int q = X.step[v];
+            const int q = step[v];
             const int na = win_entry(jb, wt, own, a), nb = win_entry(jb, wt, own, b);
             const bool later = lane >= 2 * v + 2 && lane < 2 * nv;
             const unsigned hit = __ballot_sync(0xffffffffu, later && (na >= 0 || nb >= 0));
             if (apply && later) {
-                for (int n = na; n >= 0; n = __ldg(wt.alias + n)) atomicXor(&words[n], 1u << lane);
-                for (int n = nb; n >= 0; n = __ldg(wt.alias + n)) atomicXor(&words[n], 1u << lane);
+                if (na >= 0) atomicXor(&words[na], 1u << lane);
+                if (nb >= 0) atomicXor(&words[nb], 1u << lane);
+                if (wt.aliases) {
+                    for (int n = na; n >= 0 && (n = __ldg(wt.alias + n)) >= 0;) atomicXor(&words[n], 1u << lane);
+                    for (int n = nb; n >= 0 && (n = __ldg(wt.alias + n)) >= 0;) atomicXor(&words[n], 1u << lane);
+                }
             }
             const int i = (s_w + lane) & (kWinRing - 1);
             bool eq = false;
@@ -270,7 +279,7 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
             }
             const unsigned same = __ballot_sync(0xffffffffu, eq);
             if (lane == 0) {
-                X.nbr[v] = hit ? X.step[(__ffs(hit) - 1) >> 1] : 32;
+                X.nbr[v] = hit ? step[(__ffs(hit) - 1) >> 1] : 32;
                 X.same[v] = same ? __ffs(same) - 1 : 32;
             }
         };
@@ -279,16 +288,22 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
             //    accepted flipped in the later swaps' words (XORs into zeroed words: in any order)
             const int4 own = X.site[lane];
             const int del = X.del[lane];
+            bool touched = false;
             for (int n0 = 1 + warp; n0 < n_ent; n0 += kWinBatch * nw) {      // (no row lists its own site)
                 uint32_t mine = 0;
                 int at[kWinBatch]; int8_t v[kWinBatch];
 #pragma unroll
                 for (int i = 0; i < kWinBatch; ++i) {
-                    const int4 e = n0 + i * nw < n_ent ? ent[n0 + i * nw] : ent[0];
+                    const int4 e = ent[min(n0 + i * nw, n_ent - 1)];
                     uint32_t q0 = (uint32_t)(own.x + e.x), q1 = (uint32_t)(own.y + e.y), q2 = (uint32_t)(own.z + e.z);
                     q0 = min(q0, q0 - (uint32_t)jb.d0); q1 = min(q1, q1 - (uint32_t)jb.d1); q2 = min(q2, q2 - (uint32_t)jb.d2);
                     at[i] = e.w;
                     v[i] = gsig[(q0 * (uint32_t)jb.d1 + q1) * (uint32_t)jb.d2 + q2];
+                }
+                if (!touched) {                                  // (while the loads are on their way)
+                    touched = true;
+                    for (int t = warp; t < nv; t += nw)
+                        if ((pred >> t) & 1u) touch(t, own, true);
                 }
 #pragma unroll
                 for (int i = 0; i < kWinBatch; ++i) {
@@ -297,8 +312,9 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
                 }
                 if (lane < kWinBatch && n0 + lane * nw < n_ent) atomicXor(&words[n0 + lane * nw], mine);
             }
-            for (int v = warp; v < nv; v += nw)
-                if ((pred >> v) & 1u) touch(v, own, true);
+            if (!touched)                                        // (a warp without entries)
+                for (int t = warp; t < nv; t += nw)
+                    if ((pred >> t) & 1u) touch(t, own, true);
             __syncthreads();
             // 2. rows: odd products per column and site (the last warp draws proposals: 64 steps ahead of the window's
             //    start stay drawn, whatever the window's progress; at most 128 are in the ring)
@@ -318,13 +334,13 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
                 const uint32_t s1 = v[3] ^ v[4] ^ v[5], k1 = (v[3] & v[4]) | (v[5] & (v[3] | v[4]));
                 const uint32_t w1 = s0 ^ s1 ^ v[6], k2 = (s0 & s1) | (v[6] & (s0 | s1));
                 const uint32_t w2 = k0 ^ k1 ^ k2, w4 = (k0 & k1) | (k2 & (k0 | k1));
+                uint2 sg[kWinSegs];                              // (a block has at most kWinSegs segments, padded with empty ones)
+#pragma unroll
+                for (int g = 0; g < kWinSegs; ++g) sg[g] = seg[blk * kWinSegs + g];
                 const uint32_t t1 = transpose(w1), t2 = transpose(w2), t4 = transpose(w4);
-                const int g1 = seg_off[blk + 1];
-#pragma unroll 4
-                for (int g = seg_off[blk]; g < g1; ++g) {
-                    const uint2 sg = seg[g];
-                    atomicAdd(&cnt[sg.y * 33 + lane], __popc(t1 & sg.x) + 2 * __popc(t2 & sg.x) + 4 * __popc(t4 & sg.x));
-                }
+#pragma unroll
+                for (int g = 0; g < kWinSegs; ++g)
+                    if (sg[g].x) atomicAdd(&cnt[sg[g].y + lane], __popc(t1 & sg[g].x) + 2 * __popc(t2 & sg[g].x) + 4 * __popc(t4 & sg[g].x));
             }
         }
         if (warp == nw - 1 && drawn < T && drawn < s_w + 96 && drawn + lane < T) {
@@ -339,7 +355,7 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
             for (int v = warp; v < kWinSwaps; v += nw) {
                 int32_t *ca = cnt + 2 * v, *cb = ca + 1;
                 if (v < nv) {
-                    const int i = (s_w + X.step[v]) & (kWinRing - 1);
+                    const int i = (s_w + step[v]) & (kWinRing - 1);
                     const int sgn = X.spa[v] ? -1 : 1;
                     const unsigned long long u = ring.u[i];
                     const float lnu = ring.lnu[i];
@@ -377,11 +393,12 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
         //    only at a later step that shares a site with it (once accepted); one that did not, at the first later step
         //    whose dE it moves.  (That step lies after the swap, so the least of these over all swaps of the window is
         //    the least over the decided ones.)
+        //    Warp 0 only writes the accepted swaps and lists the next window; warp 1 keeps energies, samples and counts.
         if (warp < 2) {
             long long part = 0;
             int flags = 0, q = 32, first = 32;
             if (lane < nv) {
-                flags = X.flags[lane]; q = X.step[lane]; part = X.part[lane];
+                flags = X.flags[lane]; q = step[lane];
                 const int a = flags & 1, p = (pred >> lane) & 1;
                 if (a) first = X.same[lane];
                 if (a != p) first = min(first, X.nbr[lane]);
@@ -389,22 +406,25 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
             const int limit = min(n_w, (int)__reduce_min_sync(0xffffffffu, (unsigned)first));
             const bool mine = (flags & 1) && q < limit;
             const unsigned acc = __ballot_sync(0xffffffffu, mine);
-            if (warp == 1) {                                   // tracked sums: each changed row moves its column by +-2
-                if (track)
-                    for (unsigned m = acc; m; m &= m - 1)
-                        for (int c = lane; c < n_cols; c += 32) dcv[c] += 2 * (int)nsw[(__ffs(m) - 1) * n_cols + c];
-            } else {
-                const unsigned decided = __ballot_sync(0xffffffffu, lane < nv && q < limit);
-                nnear += __popc(__ballot_sync(0xffffffffu, (flags & 2) && q < limit));
-                nacc += __popc(acc);
-                score = max(-64, min(64, score + 2 * __popc(acc) - __popc(decided)));
-                if (lane < nv && q >= limit) X.known[(s_w + q) & (kWinRing - 1)] = (flags & 1) ? 1 : 2;
+            if (warp == 0) {
                 // the two sites of each accepted swap, a lane a site
                 if ((acc >> (lane >> 1)) & 1u) {
-                    const int4 k = X.site[lane];
-                    const int sn = (lane & 1) ? X.spa[lane >> 1] : 1 - X.spa[lane >> 1];
-                    gsig[k.w] = (int8_t)sn;
+                    const int sa = X.spa[lane >> 1];
+                    gsig[X.site[lane].w] = (int8_t)((lane & 1) ? sa : 1 - sa);
                 }
+                if (lane < nv && q >= limit) X.known[(s_w + q) & (kWinRing - 1)] = (flags & 1) ? 1 : 2;
+                const unsigned decided = __ballot_sync(0xffffffffu, lane < nv && q < limit);
+                score = max(-64, min(64, score + 2 * __popc(acc) - __popc(decided)));
+                s_cur = s_w + limit;
+                __syncwarp();
+                list_window();
+            } else {
+                if (lane < nv) part = X.part[lane];
+                nnear += __popc(__ballot_sync(0xffffffffu, (flags & 2) && q < limit));
+                nacc += __popc(acc);
+                if (track)                                      // tracked sums: each changed row moves its column by +-2
+                    for (unsigned m = acc; m; m &= m - 1)
+                        for (int c = lane; c < n_cols; c += 32) dcv[c] += 2 * (int)nsw[(__ffs(m) - 1) * n_cols + c];
                 const bool sample = si > 0 && s_next <= s_w + limit;
                 long long pre = dsum; double Epre = E;          // energy after this lane's step (when sampled)
                 if (FIX) {
@@ -437,21 +457,18 @@ __global__ void __launch_bounds__(512, 2) ce_win_chunk_kernel(const __grid_const
                         jb.E_samples[(int64_t)(s1 / si - 1) * jb.R + t] = FIX ? E0 + (double)pre * fscale : Epre;
                     s_next += (s_w + limit - s_next) / si * si + si;
                 }
-                s_cur = s_w + limit;
-                __syncwarp();
-                list_window();
             }
         }
     }
-    if (FIX)                                                    // warp 0: the minimum over its lanes
+    if (FIX)                                                    // warp 1: the minimum over its lanes
         for (int o = 16; o > 0; o >>= 1) dmin = min(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
     if (track)
         for (int c = tid; c < n_cols; c += nt) jb.cv[(int64_t)r * n_cols + c] += dcv[c];
     __syncthreads();                                           // the replica's outputs are written before it is counted
-    if (tid == 0) {
+    if (tid == 32) {
         if (FIX) { E = E0 + (double)dsum * fscale; if (T > 0) Emin = fmin(Emin, E0 + (double)dmin * fscale); }
         jb.E[r] = E; jb.E_min_rep[r] = Emin; jb.n_acc[r] += nacc;
         if (jb.n_near) jb.n_near[r] += nnear;
     }
-    if (warp == 0 && jb.ex_sync) fused_chunk_end(jb, g0, lane);
+    if (warp == 1 && jb.ex_sync) fused_chunk_end(jb, g0, lane);
 }
