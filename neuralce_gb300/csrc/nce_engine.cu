@@ -158,13 +158,13 @@ __device__ __forceinline__ float patched(const NceJob &jb, int lvl, const float 
     return cache[(size_t)q * Cin + c];
 }
 
-// Tile geometry of the layer GEMM: D/4 column groups of 4 outputs, 256/(D/4) site groups, TM sites per tile,
+// Tile geometry of the layer GEMM: D/4 column groups of 4 outputs, nt/(D/4) site groups, TM sites per tile,
 // MS sites per thread (register micro-tile MS x 4).  D in {16, 32, 64, 128}.
-// Tile rows: 128 on the tcgen05 path; otherwise MS sites per thread x SG = 256 / (D / 4) site groups, MS = 4
-// (the mma.sync warp tiling needs it), on the float32 path at most 128 rows (D = 16: MS = 2)
-__host__ __device__ __forceinline__ int tile_tm(int D, int tc = 0, int mma = 0) {
-    const int SG = 256 / (D / 4);
-    return tc ? 128 : (mma ? 4 : (SG >= 64 ? 2 : 4)) * SG;
+// Tile rows: 128 on the tcgen05 path; otherwise MS sites per thread x SG = nt / (D / 4) site groups, MS = 4
+// (the mma.sync warp tiling, on 256 threads, needs it), on the float32 path at most 128 rows
+__host__ __device__ __forceinline__ int tile_tm(int D, int tc, int mma, int nt) {
+    const int SG = nt / (D / 4);
+    return tc ? 128 : (mma ? 4 : (SG >= 128 ? 1 : SG >= 64 ? 2 : 4)) * SG;
 }
 __host__ __device__ __forceinline__ int kpad16(int k) { return (k + 15) & ~15; }
 // float32 tile row stride: a multiple of 4 floats (16-byte rows for float4 reads along K) above Kin
@@ -321,7 +321,7 @@ struct LayerW {            // weights of one layer as seen by the kernel (shared
 // caches, row r N + s being site s of replica r.  Inputs come from level lvl
 // (cache patched with the step's values, or unpatched when slot == nullptr).  For every site and group of 4
 // consecutive output columns, `sink(pos, col0, v[4])` receives the activated outputs (pos < 0: padding lane); with head
-// weights ehw, tcgen05 tiles sum each site's energy themselves (head terms, then the linear term of the layer-0 row
+// weights ehw, the tiles sum each site's energy themselves (head terms, then the linear term of the layer-0 row
 // esink.row(pos, site, slot), as site_energy does) and hand it to esink.done(pos, site, energy).
 // sum over the D/4 lanes of one site (consecutive lanes of one warp)
 __device__ __forceinline__ float group_sum(float v, int ncg) {
@@ -329,21 +329,30 @@ __device__ __forceinline__ float group_sum(float v, int ncg) {
     return v;
 }
 
+// whether the tiles sum site energies themselves: every layer-0 channel of a site must be in flight at once (four a lane; the
+// 18 channels on the four lanes of a width-16 site took 10% longer than a sink a site); the mma.sync form keeps its sink
+constexpr int kEnergyCh = 4;
+__device__ __forceinline__ bool tile_energies(const NceDev &m) { return m.mma != 1 && m.mma != 3 && m.C0 <= kEnergyCh * (m.D / 4); }
+
 struct NoSink {
     __device__ const float *row(int64_t, int32_t, int32_t) const { return nullptr; }
     __device__ void done(int64_t, int32_t, float) const {}
 };
 
-template <typename Sink, typename ESink = NoSink>
+// (TC: the tcgen05 tiles, tc set.  The two forms are compiled apart: in one body the float32 form of the shipped model ran 10%
+// slower, 2,306 -> 2,580 us for 40 steps of 32 replicas)
+template <bool TC, typename Sink, typename ESink = NoSink>
 __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const float *cache, const float *newl, const int32_t *slot,
                             int32_t nlev, const int32_t *list, int64_t pos0, int64_t cnt, const int64_t *direct0, float *X,
-                            int32_t *src, Sink sink, int tile_begin = 0, int tile_stride = 1, TcCtx *tc = nullptr,
+                            int32_t *src, Sink sink, int tile_begin, int tile_stride, TcCtx *tc_ctx,
                             const float *ehw = nullptr, const float *lin = nullptr, ESink esink = ESink{}) {
+    TcCtx *const tc = TC ? tc_ctx : nullptr;
+    if (TC) __builtin_assume(tc != nullptr);
     const NceDev &m = jb.m;
     const int Cin = lvl == 0 ? m.C0 : m.D, D = m.D, P = m.P, W = m.W;
     const int Kin = (1 + P) * Cin, XS = x_stride(Kin);
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int ncg = D / 4, SG = (tc ? nt : 256) / ncg, TM = tile_tm(D, tc != nullptr, m.mma), MS = TM / SG;
+    const int ncg = D / 4, SG = nt / ncg, TM = tile_tm(D, tc != nullptr, m.mma, nt), MS = TM / SG;
     const int cg = tid % ncg, sg = tid / ncg;
     const int PW = 1 + P * W;
     // row of each site and shell partner: the step's new value, the cache, or a row of zeros (masked partner)
@@ -396,6 +405,35 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
         } else {
             X[(size_t)ms * XS + k] = v0; X[(size_t)ms * XS + k + 1] = v1;
         }
+    };
+    // energies of four sites of the tile (rows mm) from this lane's head terms: the linear layer-0 term with the four rows in
+    // flight (kEnergyCh channels a lane), the group sum, and the total left in etot (over tinv, dead
+    // by then), which one thread a site hands on: the loads behind a site's end then overlap over all sites
+    constexpr int LC = kEnergyCh;
+    float *etot = tinv;
+    auto energies = [&](int64_t t0, int tm, const int mm[4], float part[4]) {
+        const float *hr[4];
+        float x[4][LC], lv[LC];
+#pragma unroll
+        for (int j = 0; j < LC; ++j) lv[j] = cg + j * ncg < m.C0 ? lin[cg + j * ncg] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int mc = mm[i] < tm ? mm[i] : 0;
+            hr[i] = esink.row(mm[i] < tm ? t0 + mm[i] : -1, tsite[mc], tslot[mc]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < LC; ++j) x[i][j] = cg + j * ncg < m.C0 ? hr[i][cg + j * ncg] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int j = 0; j < LC; ++j) if (cg + j * ncg < m.C0) part[i] = fmaf(x[i][j], lv[j], part[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) part[i] = group_sum(part[i], ncg);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) if (cg == 0 && mm[i] < tm) etot[mm[i]] = part[i];
     };
     for (int64_t t0 = (int64_t)tile_begin * TM; t0 < cnt; t0 += (int64_t)tile_stride * TM) {
         const int tm = (int)min((int64_t)TM, cnt - t0);
@@ -687,41 +725,17 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
                 }
             }
             if (ehw) {
-                // the linear layer-0 term: four sites' rows in flight (at most four channels a lane; wider ones in a loop)
-                constexpr int LC = 4;
-                float lv[LC];
-#pragma unroll
-                for (int j = 0; j < LC; ++j) lv[j] = cg + j * ncg < m.C0 ? lin[cg + j * ncg] : 0.f;
                 for (int i0 = 0; i0 < MS; i0 += 4) {
-                    const float *hr[4];
-                    float x[4][LC];
+                    int mm[4]; float part[4];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int mm = sg + min(i0 + i, MS - 1) * SG, mc = mm < tm ? mm : 0;
-                        hr[i] = esink.row(mm < tm ? t0 + mm : -1, tsite[mc], tslot[mc]);
+                    for (int i = 0; i < 4; ++i) {                // (repeated rows past the last: the same total again)
+                        mm[i] = sg + min(i0 + i, MS - 1) * SG;
+                        part[i] = Y[mm[i] * YS + cg];
                     }
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-#pragma unroll
-                        for (int j = 0; j < LC; ++j) x[i][j] = cg + j * ncg < m.C0 ? hr[i][cg + j * ncg] : 0.f;
-                    float tot[4];
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int mm = sg + min(i0 + i, MS - 1) * SG;
-                        float part = Y[mm * YS + cg];
-#pragma unroll
-                        for (int j = 0; j < LC; ++j) if (cg + j * ncg < m.C0) part = fmaf(x[i][j], lv[j], part);
-                        for (int c = cg + LC * ncg; c < m.C0; c += ncg) part = fmaf(hr[i][c], lin[c], part);
-                        tot[i] = part;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) tot[i] = group_sum(tot[i], ncg);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int mm = sg + min(i0 + i, MS - 1) * SG;
-                        if (i0 + i < MS && mm < tm && cg == 0) esink.done(t0 + mm, tsite[mm], tot[i]);
-                    }
+                    energies(t0, tm, mm, part);
                 }
+                __syncthreads();
+                if (tid < tm) esink.done(t0 + tid, tsite[tid], etot[tid]);
             }
             __syncthreads();
             continue;
@@ -813,8 +827,8 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
             o[i][0] = b4.x; o[i][1] = b4.y; o[i][2] = b4.z; o[i][3] = b4.w;
             g[i][0] = gb4.x; g[i][1] = gb4.y; g[i][2] = gb4.z; g[i][3] = gb4.w;
         }
-        // rows sg + i SG, i < MS (MS = 2: the last two micro-tile rows repeat the first two and are not used)
-        const float *x0 = X + (size_t)sg * XS, *x1 = x0 + (size_t)SG * XS;
+        // rows sg + i SG, i < MS (fewer than four: the last micro-tile rows repeat the first ones and are not used)
+        const float *x0 = X + (size_t)sg * XS, *x1 = MS > 1 ? x0 + (size_t)SG * XS : x0;
         const float *x2 = MS > 2 ? x1 + (size_t)SG * XS : x0, *x3 = MS > 2 ? x2 + (size_t)SG * XS : x1;
         auto fma16 = [&](float v0, float v1, float v2, float v3, const float4 w4) {
             o[0][0] = fmaf(v0, w4.x, o[0][0]); o[0][1] = fmaf(v0, w4.y, o[0][1]); o[0][2] = fmaf(v0, w4.z, o[0][2]); o[0][3] = fmaf(v0, w4.w, o[0][3]);
@@ -847,16 +861,37 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
             }
         }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            if (i < MS) {
-                const int mm = sg + i * SG;
-                float v[4];
+        for (int i = 0; i < 4; ++i)
+            if (i < MS)
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     float a = act_fn(m.act, o[i][q]);
                     if (LW.G) a *= 1.0f / (1.0f + expf(-g[i][q]));
-                    v[q] = a;
+                    o[i][q] = a;
                 }
+        if (ehw) {
+            int mm[4]; float part[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {                        // (repeated rows past the last: the same total again)
+                const int k = i < MS ? i : 0;
+                mm[i] = sg + k * SG;
+                float a = 0.f;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) a = fmaf(i < MS ? o[i][q] : o[0][q], ehw[cg * 4 + q], a);
+                part[i] = a;
+            }
+            __syncthreads();                                     // (the gather's reads of tinv are over)
+            energies(t0, tm, mm, part);
+            __syncthreads();
+            if (tid < tm) esink.done(t0 + tid, tsite[tid], etot[tid]);
+            __syncthreads();
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (i < MS) {
+                const int mm = sg + i * SG;
+                const float v[4] = {o[i][0], o[i][1], o[i][2], o[i][3]};
                 sink(mm < tm ? t0 + mm : -1, cg * 4, v, tsite[mm < tm ? mm : 0], tslot[mm < tm ? mm : 0]);
             }
         }
@@ -895,7 +930,7 @@ __device__ __forceinline__ void csync() {
     if (CLUSTER) { __threadfence(); cg::this_cluster().sync(); } else { __syncthreads(); }
 }
 
-template <bool CLUSTER>
+template <bool CLUSTER, bool TC>
 __device__ void nce_step(const NceJob &jb, int r, int t, int64_t s_idx, NceCtl &ctl, unsigned long long *dh, float *X,
                          int32_t *src, const LayerW *LWs, const float *lin, const float *hw, int32_t *ent_site, int32_t *ent_pos,
                          int8_t *ent_sig, double &E, int64_t &nacc, int64_t &nnear, const NceCtx &cx, TcCtx *tc) {
@@ -1184,7 +1219,7 @@ __device__ void nce_step(const NceJob &jb, int r, int t, int64_t s_idx, NceCtl &
         if (lvl + 1 < L) {
             float *outb = level_buf(jb, nb, lvl + 1);
             const int D = m.D;
-            layer_tiles(jb, lvl, LWs[lvl], cache, newl, slot, ctl.nl[lvl], list, 0, nout, nullptr, X, src,
+            layer_tiles<TC>(jb, lvl, LWs[lvl], cache, newl, slot, ctl.nl[lvl], list, 0, nout, nullptr, X, src,
                         [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
                             if (pos >= 0) *reinterpret_cast<float4 *>(outb + (size_t)pos * D + c0) = make_float4(v[0], v[1], v[2], v[3]);
                         }, rank, CL, tc);
@@ -1204,11 +1239,11 @@ __device__ void nce_step(const NceJob &jb, int r, int t, int64_t s_idx, NceCtl &
                 en_r[pos] = ev;
                 dloc += (unsigned long long)llrint(((double)ev - (double)e_r[site]) * kFix);
             };
-            layer_tiles(jb, lvl, LWs[lvl], cache, newl, slot, ctl.nl[lvl], list, 0, nout, nullptr, X, src,
+            layer_tiles<TC>(jb, lvl, LWs[lvl], cache, newl, slot, ctl.nl[lvl], list, 0, nout, nullptr, X, src,
                         [&](int64_t pos, int c0, const float *v, int32_t site, int32_t p0) {
                             const float tot = site_energy(v, c0, hw, pos >= 0 ? row(pos, site, p0) : nullptr, lin, m.C0, ncg);
                             if (pos >= 0 && c0 == 0) done(pos, site, tot);
-                        }, rank, CL, tc, tc ? hw : nullptr, lin, EnergySink<decltype(row), decltype(done)>{row, done});
+                        }, rank, CL, tc, tile_energies(m) ? hw : nullptr, lin, EnergySink<decltype(row), decltype(done)>{row, done});
         }
     }
     if (L == 0) {
@@ -1320,11 +1355,11 @@ __host__ __device__ inline size_t weight_floats(int depth, int P, int C0, int D,
 // A operand(s) [128][tc_ks] or float32 output rows [128][min(D, kTcCols) + 4], whichever is larger.
 struct SmemPlan {
     size_t dh, X, src, wt, ent, w, dh_bytes, tile_end, total_w;
-    __host__ __device__ static SmemPlan make(const NceDev &m, bool with_dh = true) {
+    __host__ __device__ static SmemPlan make(const NceDev &m, int nt, bool with_dh = true) {
         auto al = [](size_t x) { return (x + 15) / 16 * 16; };
         auto al128 = [](size_t x) { return (x + 127) / 128 * 128; };
         SmemPlan p;
-        const int TM = tile_tm(m.D, m.tc, m.mma), Kmax = tile_kin(m.P, m.C0, m.D);
+        const int TM = tile_tm(m.D, m.tc, m.mma, nt), Kmax = tile_kin(m.P, m.C0, m.D);
         // layer-0 change per (site, channel): int32 counts for +-1 point functions, int64 fixed point otherwise
         p.dh_bytes = with_dh ? al((m.l0bin ? sizeof(int32_t) : sizeof(unsigned long long)) * (size_t)m.n0max * m.C0) : 0;
         p.X = 0;
@@ -1347,14 +1382,14 @@ struct SmemPlan {
 
 // MINB = CTAs resident per SM: 1 (all registers) or 2 (at most 128 registers a thread, twice the warps to hide
 // the latency of the gathers and barriers when two CTAs' shared memory fits an SM)
-template <int MINB, int NT>
+template <int MINB, int NT, bool TC>
 __global__ void __launch_bounds__(NT, MINB) nce_chunk_kernel(const __grid_constant__ NceJob jb, int32_t w_smem) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ NceCtl ctl;
     const int r = blockIdx.x;
     if (r >= jb.R) return;
     const NceDev &m = jb.m;
-    const SmemPlan sp = SmemPlan::make(m);
+    const SmemPlan sp = SmemPlan::make(m, NT);
     unsigned long long *dh = reinterpret_cast<unsigned long long *>(smem + sp.dh);
     float *X = reinterpret_cast<float *>(smem + sp.X);
     int32_t *src = reinterpret_cast<int32_t *>(smem + sp.src);
@@ -1367,23 +1402,23 @@ __global__ void __launch_bounds__(NT, MINB) nce_chunk_kernel(const __grid_consta
     __shared__ __align__(8) uint64_t tc_mbar[2];
     __shared__ uint32_t tc_slot;
     TcCtx tcx;
-    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
+    if (TC) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
     const int t = jb.slot_of_rep[r];
     double E = jb.E[r];
     int64_t nacc = 0, nnear = 0;
     NceCtx cx; cx.rank = 0; cx.CL = 1; cx.lctl = &ctl;
     for (int64_t s = 0; s < jb.n_steps; ++s) {
-        nce_step<false>(jb, r, t, s, ctl, dh, X, src, lw, lin, hw, ent_site, ent_pos, ent_sig, E, nacc, nnear, cx, m.tc ? &tcx : nullptr);
+        nce_step<false, TC>(jb, r, t, s, ctl, dh, X, src, lw, lin, hw, ent_site, ent_pos, ent_sig, E, nacc, nnear, cx, TC ? &tcx : nullptr);
         if (threadIdx.x == 0 && jb.E_samples && (s + 1) % jb.sample_interval == 0)
             jb.E_samples[((s + 1) / jb.sample_interval - 1) * jb.R + t] = E;
         __syncthreads();
     }
     if (threadIdx.x == 0) { jb.E[r] = E; jb.n_acc[r] += nacc; if (jb.n_near) jb.n_near[r] += nnear; }
-    if (m.tc) tc_end(m.D, tcx);
+    if (TC) tc_end(m.D, tcx);
 }
 
 // the same chunk with each replica spread over a thread-block cluster of gridDim.x / R CTAs
-template <int MINB, int NT>
+template <int MINB, int NT, bool TC>
 __global__ void __launch_bounds__(NT, MINB) nce_chunk_cluster_kernel(const __grid_constant__ NceJob jb, int32_t w_smem) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ NceCtl ctl;
@@ -1392,7 +1427,7 @@ __global__ void __launch_bounds__(NT, MINB) nce_chunk_cluster_kernel(const __gri
     const int r = blockIdx.x / CL;
     if (r >= jb.R) return;                           // whole clusters only: gridDim.x == R * CL
     const NceDev &m = jb.m;
-    const SmemPlan sp = SmemPlan::make(m);
+    const SmemPlan sp = SmemPlan::make(m, NT);
     unsigned long long *dh = reinterpret_cast<unsigned long long *>(smem + sp.dh);
     float *X = reinterpret_cast<float *>(smem + sp.X);
     int32_t *src = reinterpret_cast<int32_t *>(smem + sp.src);
@@ -1405,20 +1440,20 @@ __global__ void __launch_bounds__(NT, MINB) nce_chunk_cluster_kernel(const __gri
     __shared__ __align__(8) uint64_t tc_mbar[2];
     __shared__ uint32_t tc_slot;
     TcCtx tcx;
-    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
+    if (TC) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
     NceCtx cx; cx.rank = rank; cx.CL = CL; cx.lctl = cluster.map_shared_rank(&ctl, 0);
     cluster.sync();
     const int t = jb.slot_of_rep[r];
     double E = jb.E[r];
     int64_t nacc = 0, nnear = 0;
     for (int64_t s = 0; s < jb.n_steps; ++s) {
-        nce_step<true>(jb, r, t, s, ctl, dh, X, src, lw, lin, hw, ent_site, ent_pos, ent_sig, E, nacc, nnear, cx, m.tc ? &tcx : nullptr);
+        nce_step<true, TC>(jb, r, t, s, ctl, dh, X, src, lw, lin, hw, ent_site, ent_pos, ent_sig, E, nacc, nnear, cx, TC ? &tcx : nullptr);
         if (rank == 0 && threadIdx.x == 0 && jb.E_samples && (s + 1) % jb.sample_interval == 0)
             jb.E_samples[((s + 1) / jb.sample_interval - 1) * jb.R + t] = E;
     }
     if (rank == 0 && threadIdx.x == 0) { jb.E[r] = E; jb.n_acc[r] += nacc; if (jb.n_near) jb.n_near[r] += nnear; }
     cluster.sync();                                   // no CTA leaves while others may still read its shared memory
-    if (m.tc) tc_end(m.D, tcx);
+    if (TC) tc_end(m.D, tcx);
 }
 
 // Commit of the swaps kept by a force = -2 chunk (nce_nce_local_delta): one CTA per replica writes the new layer-0,
@@ -1673,36 +1708,36 @@ __global__ void nce_h0_kernel(NceDev m, const int8_t *sigma, int32_t R, float *h
 // of the last layer.  One launch takes every replica's tiles, a CTA tiles blockIdx.x, blockIdx.x + gridDim.x, ...: a
 // launch per replica and layer left most SMs idle on small cells (2,048 sites x 32
 // replicas, float32 width 64, whole cache: 2,340 -> 724 us; 131,072 x 8, split bf16 width 128: 10.4 -> 9.5 ms)
-template <int MINB, int NT>
+template <int MINB, int NT, bool TC>
 __global__ void __launch_bounds__(NT, MINB) nce_layer_all_kernel(const __grid_constant__ NceJob jb, int lvl, const float *in, float *out,
                                                                  float *__restrict__ e_out, int64_t rows) {
     extern __shared__ __align__(16) unsigned char smem[];
     const NceDev &m = jb.m;
-    const SmemPlan sp = SmemPlan::make(m, false);
+    const SmemPlan sp = SmemPlan::make(m, NT, false);
     float *X = reinterpret_cast<float *>(smem + sp.X);
     int32_t *src = reinterpret_cast<int32_t *>(smem + sp.src);
     __shared__ __align__(8) uint64_t tc_mbar[2];
     __shared__ uint32_t tc_slot;
     TcCtx tcx;
-    if (m.tc) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
-    TcCtx *tcp = m.tc ? &tcx : nullptr;
+    if (TC) tc_begin(m.D, tcx, smem + sp.wt, tc_mbar, &tc_slot);
+    TcCtx *tcp = TC ? &tcx : nullptr;
     const float *__restrict__ h0 = jb.h0;
     const int64_t row0 = 0;
     const int D = m.D, ncg = D / 4;
     LayerW LW; LW.W = m.Wc[lvl]; LW.b = m.bias[lvl]; LW.G = m.gate ? m.G[lvl] : nullptr; LW.gb = m.gate ? m.gb[lvl] : nullptr;
     if (out) {
-        layer_tiles(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, rows, &row0, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
+        layer_tiles<TC>(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, rows, &row0, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
             if (pos >= 0) *reinterpret_cast<float4 *>(out + (size_t)pos * D + c0) = make_float4(v[0], v[1], v[2], v[3]);
         }, blockIdx.x, gridDim.x, tcp);
     } else {
         auto row = [&](int64_t pos, int32_t, int32_t) -> const float * { return pos >= 0 ? h0 + (size_t)pos * m.C0 : m.zrow; };
         auto done = [&](int64_t pos, int32_t, float tot) { e_out[pos] = (m.Mb[pos % m.nB] > 1) ? tot : 0.f; };
-        layer_tiles(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, rows, &row0, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
+        layer_tiles<TC>(jb, lvl, LW, in, nullptr, nullptr, 0, nullptr, 0, rows, &row0, X, src, [&](int64_t pos, int c0, const float *v, int32_t, int32_t) {
             const float tot = site_energy(v, c0, m.head_w, pos >= 0 ? h0 + (size_t)pos * m.C0 : nullptr, m.lin, m.C0, ncg);
             if (pos >= 0 && c0 == 0) done(pos, 0, tot);
-        }, blockIdx.x, gridDim.x, tcp, tcp ? m.head_w : nullptr, m.lin, EnergySink<decltype(row), decltype(done)>{row, done});
+        }, blockIdx.x, gridDim.x, tcp, tile_energies(m) ? m.head_w : nullptr, m.lin, EnergySink<decltype(row), decltype(done)>{row, done});
     }
-    if (m.tc) tc_end(m.D, tcx);
+    if (TC) tc_end(m.D, tcx);
 }
 
 __global__ void nce_e0_kernel(NceDev m, const float *h0, int64_t n, float *e) {
@@ -1764,12 +1799,12 @@ constexpr size_t kStepSmemMax = 232448 - 1024;
 // two CTAs per SM: 228 KB of shared memory per SM, less 1 KB reserved per CTA and the static shared memory
 constexpr size_t kStepSmemMax2 = 233472 / 2 - 2048;
 
-static size_t tile_smem(const NceDev &m) {
-    return SmemPlan::make(m, false).tile_end;
+static size_t tile_smem(const NceDev &m, int nt) {
+    return SmemPlan::make(m, nt, false).tile_end;
 }
 
-static size_t step_smem(const NceDev &m, bool w_smem) {
-    const SmemPlan p = SmemPlan::make(m);
+static size_t step_smem(const NceDev &m, bool w_smem, int nt) {
+    const SmemPlan p = SmemPlan::make(m, nt);
     return w_smem ? p.total_w : p.w;
 }
 
@@ -1797,22 +1832,30 @@ static int launch_steps(nce_nce_model *h, const NceJob &jb, int cluster, int cta
     const int per_sm = ctas_per_sm > 1 ? ctas_per_sm : 1;
     NCE_CHECK(per_sm <= 2, "nce_nce_run_chunk: ctas_per_sm must be 1 or 2");
     const size_t lim = per_sm == 2 ? kStepSmemMax2 : kStepSmemMax;
-    const bool w_smem = step_smem(h->dev, true) <= lim;
-    const size_t sm = step_smem(h->dev, w_smem);
+    // A CTA with an SM of its own: 512 threads, twice the partner rows in flight per tile (tensor-core forms: 55,296 sites x 16,
+    // width 128 split, 12 steps 3.39 -> 1.77 ms with the gather and the epilogue of the tiles; float32
+    // width 64, 2,048 sites x 32, 25 steps: 3.99 -> 3.19 ms with the energies of a tile in flight together and the forms compiled
+    // apart; width 16, whose tile stays at 128 sites, lost 2%).  float32 tiles grow with the threads: 256 where only
+    // those leave room for the weights.
+    const NceDev &dv = h->dev;
+    int nt = per_sm == 1 && (dv.tc || (dv.mma == 0 && dv.D >= 32)) ? 512 : 256;
+    if (nt == 512 && !dv.tc && step_smem(dv, true, 512) > lim && (step_smem(dv, true, 256) <= lim || step_smem(dv, false, 512) > lim)) nt = 256;
+    const bool w_smem = step_smem(dv, true, nt) <= lim;
+    const size_t sm = step_smem(dv, w_smem, nt);
     NCE_CHECK(per_sm == 1 || !h->dev.tc || h->dev.D <= 64, "nce_nce_run_chunk: tensor-core tiles of width 128 do not fit 2 CTAs per SM");
     NCE_CHECK(sm <= lim, "nce_nce_run_chunk: %zu bytes of shared memory per CTA do not fit %d CTAs per SM", sm, per_sm);
     const int CL = cluster > 1 ? cluster : 1;
     NCE_CHECK(CL == 1 || CL == 2 || CL == 4 || CL == 8, "nce_nce_run_chunk: cluster must be 1, 2, 4 or 8");
-    // tensor-core forms with an SM of their own: 512 threads, twice the partner rows in flight per tile (55,296 sites x 16,
-    // width 128 split, 12 steps: 3.39 -> 1.77 ms with the gather and the epilogue of the tiles)
-    const bool wide = h->dev.tc && per_sm == 1;
-    const int nt = wide ? 512 : 256;
+    const bool wide = nt == 512;
     if (CL == 1 || h->dev.depth == 0) {
-        auto kern = per_sm == 2 ? nce_chunk_kernel<2, 256> : wide ? nce_chunk_kernel<1, 512> : nce_chunk_kernel<1, 256>;
+        auto kern = dv.tc ? (wide ? nce_chunk_kernel<1, 512, true> : nce_chunk_kernel<2, 256, true>)
+                          : per_sm == 2 ? nce_chunk_kernel<2, 256, false> : wide ? nce_chunk_kernel<1, 512, false> : nce_chunk_kernel<1, 256, false>;
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
         kern<<<jb.R, nt, sm, stream>>>(jb, w_smem ? 1 : 0);
     } else {
-        auto kern = per_sm == 2 ? nce_chunk_cluster_kernel<2, 256> : wide ? nce_chunk_cluster_kernel<1, 512> : nce_chunk_cluster_kernel<1, 256>;
+        auto kern = dv.tc ? (wide ? nce_chunk_cluster_kernel<1, 512, true> : nce_chunk_cluster_kernel<2, 256, true>)
+                          : per_sm == 2 ? nce_chunk_cluster_kernel<2, 256, false>
+                          : wide ? nce_chunk_cluster_kernel<1, 512, false> : nce_chunk_cluster_kernel<1, 256, false>;
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
         cudaLaunchConfig_t cfg; std::memset(&cfg, 0, sizeof(cfg));
         cfg.gridDim = dim3((unsigned)(jb.R * CL)); cfg.blockDim = dim3(nt); cfg.dynamicSmemBytes = sm;
@@ -2188,9 +2231,10 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
         if (e == cudaSuccess) e = cudaMemset(h->err, 0, sizeof(int32_t));
         if (e != cudaSuccess) rc = fail(NCE_ERR_CUDA, "nce_nce_create: %s", cudaGetErrorString(e));
     }
-    if (!rc && step_smem(m, false) > kStepSmemMax)
+    const int nt_min = m.tc ? 512 : 256;
+    if (!rc && step_smem(m, false, nt_min) > kStepSmemMax)
         rc = fail(NCE_ERR_UNSUPPORTED, "nce_nce_create: receptive field%s too large for shared memory (%zu bytes)",
-                  m.tc ? " and tensor-core tiles" : "", step_smem(m, false));
+                  m.tc ? " and tensor-core tiles" : "", step_smem(m, false, nt_min));
     if (rc) {
         for (void *p : h->allocs) cudaFree(p);
         delete h;
@@ -2254,11 +2298,12 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
     }
     NCE_CUDA(cudaGetLastError());
     NceJob jb = make_nce_job(h, st);
-    const size_t xs = tile_smem(m);
     // two CTAs per SM where their tiles fit (the gathers of one hide behind the other's contraction)
-    const bool two = xs <= kStepSmemMax2 && !(m.tc && m.D > 64);
+    const bool two = tile_smem(m, 256) <= kStepSmemMax2 && !(m.tc && m.D > 64);
     const int layer_nt = m.tc && !two ? 512 : 256;
-    auto layer_kern = two ? nce_layer_all_kernel<2, 256> : m.tc ? nce_layer_all_kernel<1, 512> : nce_layer_all_kernel<1, 256>;
+    const size_t xs = tile_smem(m, layer_nt);
+    auto layer_kern = m.tc ? (two ? nce_layer_all_kernel<2, 256, true> : nce_layer_all_kernel<1, 512, true>)
+                           : (two ? nce_layer_all_kernel<2, 256, false> : nce_layer_all_kernel<1, 256, false>);
     NCE_CUDA(::nce::raise_smem_limit((const void *)layer_kern, xs));
     int dev = 0, n_sm = 152;
     cudaGetDevice(&dev);
@@ -2269,7 +2314,7 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
     }
     // hidden layers: hmid[l-1] for l = 1..depth-1, then the last layer into e; all replicas' rows in one launch each (rows
     // below 2^31: more replicas take further launches)
-    const int64_t TM = tile_tm(m.D, m.tc, m.mma), rep_per = std::max<int64_t>(1, ((1ll << 31) - 1) / m.N);
+    const int64_t TM = tile_tm(m.D, m.tc, m.mma, layer_nt), rep_per = std::max<int64_t>(1, ((1ll << 31) - 1) / m.N);
     for (int l = 0; l < m.depth; ++l) {
         for (int64_t r = 0; r < st->R; r += rep_per) {
             const int64_t rows = std::min<int64_t>(rep_per, st->R - r) * m.N, tiles = (rows + TM - 1) / TM;
