@@ -2483,14 +2483,21 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                         oth = std::max(oth, (int)rel.size() - 1);
                     }
                 m->bw_oth = oth <= 3 ? 3 : 7;
+                for (int b = 0; b < t->nB; ++b) {
+                    std::map<Mem, int> at;
+                    for (const auto &col : inst[b]) for (const auto &rel : col) if (!rel.empty()) at[rel[0]] = 0;
+                    // several point-function columns on one basis site: a row anchored on another than the first XORs the first
+                    // away and its own in (two more words)
+                    if (at.size() > 1) m->bw_oth = 7;
+                    if (oth + (at.size() > 1 ? 2 : 0) > 7) bin = false;
+                }
                 std::vector<uint4> words; std::vector<int32_t> word_off(1, 0), grp_off(1, 0);
                 std::vector<uint32_t> idx, info;                 // (groups, 3, bw_oth + 1) word indices; column | rows << 16
                 for (int b = 0; b < t->nB && bin; ++b) {
                     std::map<Mem, int> at;                       // the anchor's own words first, the others by row
                     for (const auto &col : inst[b]) for (const auto &rel : col) if (!rel.empty()) at[rel[0]] = 0;
-                    if (at.size() > 1) bin = false;              // (a basis site carries one point-function column)
                     std::vector<Mem> order;
-                    for (const auto &kv : at) order.push_back(kv.first);
+                    for (const auto &kv : at) order.push_back(kv.first);       // (word 0: the first anchor)
                     if (order.empty()) order.push_back({0, 0, 0, 0});
                     std::map<Mem, int> rest;
                     for (const auto &col : inst[b]) for (const auto &rel : col) for (const auto &x : rel) if (!at.count(x)) rest[x] = 0;
@@ -2511,8 +2518,12 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                                 std::vector<uint32_t> w((size_t)m->bw_oth + 1, zero);
                                 // a missing row, or one without sign changes, XORs the anchor away
                                 if (h >= nr || inst[b][c][q + h].empty()) w[0] = 0;
-                                else
-                                    for (size_t k = 1; k < inst[b][c][q + h].size(); ++k) w[k - 1] = (uint32_t)ix[inst[b][c][q + h][k]];
+                                else {
+                                    const auto &rel = inst[b][c][q + h];
+                                    size_t n = 0;
+                                    for (size_t k = 1; k < rel.size(); ++k) w[n++] = (uint32_t)ix[rel[k]];
+                                    if (ix[rel[0]] != 0) { w[n++] = 0; w[n++] = (uint32_t)ix[rel[0]]; }
+                                }
                                 idx.insert(idx.end(), w.begin(), w.end());
                             }
                         }

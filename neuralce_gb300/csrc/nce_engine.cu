@@ -2232,6 +2232,22 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
         if (e != cudaSuccess) rc = fail(NCE_ERR_CUDA, "nce_nce_create: %s", cudaGetErrorString(e));
     }
     const int nt_min = m.tc ? 512 : 256;
+    if (!rc && m.tc) {
+        // the interface's limit on tensor-core models, wider than what the tiles need now: the whole A operand, or half of
+        // its K extent where every layer divides into halves, and all output columns beside the B operand
+        const SmemPlan p = SmemPlan::make(m, nt_min);
+        const int kp = kpad16(tile_kin(m.P, m.C0, m.D));
+        bool halves = kp % 32 == 0;
+        for (int l = 0; l < m.depth; ++l) {
+            const int kl = kpad16((1 + m.P) * (l == 0 ? m.C0 : m.D));
+            halves = halves && (kl <= kp / 2 || kl % (kp / 2) == 0);
+        }
+        auto size = [&](int ks) {
+            return p.w - p.src + std::max((size_t)128 * ks * 2 * (m.tc_split ? 2 : 1), sizeof(float) * 128 * (size_t)(m.D + 4));
+        };
+        if (size(kp) > kStepSmemMax && !(halves && size(kp / 2) <= kStepSmemMax))
+            rc = fail(NCE_ERR_UNSUPPORTED, "nce_nce_create: receptive field and tensor-core tiles too large for shared memory (%zu bytes)", size(kp));
+    }
     if (!rc && step_smem(m, false, nt_min) > kStepSmemMax)
         rc = fail(NCE_ERR_UNSUPPORTED, "nce_nce_create: receptive field%s too large for shared memory (%zu bytes)",
                   m.tc ? " and tensor-core tiles" : "", step_smem(m, false, nt_min));
@@ -2262,33 +2278,33 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
     cudaStream_t s = (cudaStream_t)stream;
     const NceDev &m = h->dev;
     const int64_t tot = (int64_t)st->R * m.N;
-    if (m.h0bits && st->R <= 65535) {
+    const int64_t items = (int64_t)m.d0 * m.d1 * ((m.d2 + 31) / 32), blocks = (items + 31) / 32;
+    int dv = 0, nsm = 152;
+    cudaGetDevice(&dv);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dv);
+    // channels in slices: enough warps for the SMs (every slice fetches the words again), counts that fit beside the words
+    int S = 1, lut_max = 0;
+    size_t sm = 0;
+    for (; m.h0bits; S *= 2) {
+        int nch = 0;
+        lut_max = 0;
+        for (int b = 0; b < m.nB; ++b)
+            for (int sl = 0; sl < S; ++sl) {
+                const int32_t *g = &h->h0grp[(size_t)b * (m.C0 + 1)], *lo = &h->h0lut_off[(size_t)b * (m.C0 + 1)];
+                const int ca = h0_first_channel(g, m.C0, sl, S), cb = sl + 1 == S ? m.C0 : h0_first_channel(g, m.C0, sl + 1, S);
+                nch = std::max(nch, cb - ca);
+                if (cb > ca) lut_max = std::max(lut_max, (lo[cb] - lo[ca] + 3) & ~3);
+            }
+        sm = sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1) + sizeof(float) * lut_max + (size_t)32 * nch * 36 * (m.h0_wide ? 2 : 1);
+        if (S >= 16 || (int64_t)m.nB * S * 2 > 65535 || (sm <= 100 * 1024 && blocks * m.nB * st->R * S >= 8ll * nsm)) break;
+    }
+    if (m.h0bits && st->R <= 65535 && sm <= 200 * 1024) {
         const int32_t W2 = (2 * m.d2 + 31) / 32 + 1;
         StreamScratch planes;
         NCE_CUDA(planes.alloc(sizeof(uint32_t) * (size_t)st->R * m.nB * m.d0 * m.d1 * W2, s));
         const int64_t prow = (int64_t)st->R * m.nB * m.d0 * m.d1;
         nce_plane_kernel<<<(int)std::min<int64_t>((prow + 7) / 8, 1 << 20), 256, 0, s>>>(m, st->sigma, st->R, W2, (uint32_t *)planes.p);
         NCE_CUDA(cudaGetLastError());
-        const int64_t items = (int64_t)m.d0 * m.d1 * ((m.d2 + 31) / 32), blocks = (items + 31) / 32;
-        int dv = 0, nsm = 152;
-        cudaGetDevice(&dv);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dv);
-        // channels in slices: enough warps for the SMs (every slice fetches the words again), counts that fit beside the words
-        int S = 1, lut_max = 0;
-        size_t sm = 0;
-        for (;; S *= 2) {
-            int nch = 0;
-            lut_max = 0;
-            for (int b = 0; b < m.nB; ++b)
-                for (int sl = 0; sl < S; ++sl) {
-                    const int32_t *g = &h->h0grp[(size_t)b * (m.C0 + 1)], *lo = &h->h0lut_off[(size_t)b * (m.C0 + 1)];
-                    const int ca = h0_first_channel(g, m.C0, sl, S), cb = sl + 1 == S ? m.C0 : h0_first_channel(g, m.C0, sl + 1, S);
-                    nch = std::max(nch, cb - ca);
-                    if (cb > ca) lut_max = std::max(lut_max, (lo[cb] - lo[ca] + 3) & ~3);
-                }
-            sm = sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1) + sizeof(float) * lut_max + (size_t)32 * nch * 36 * (m.h0_wide ? 2 : 1);
-            if (S >= 16 || (sm <= 100 * 1024 && blocks * m.nB * st->R * S >= 8ll * nsm)) break;
-        }
         auto kern = m.h0_wide ? (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 13, uint16_t> : nce_h0_bits_kernel<7, 13, uint16_t>)
                               : (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 8, uint8_t> : nce_h0_bits_kernel<7, 8, uint8_t>);
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
