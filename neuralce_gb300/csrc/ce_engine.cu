@@ -1882,8 +1882,15 @@ static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *st
     // step-by-step kernels, which keep the other tables (several basis sites, larger orders, one-cell images).
     bool use_win = use_bin;
     for (int j = 0; j < n_jobs; ++j) use_win = use_win && hs[j]->win != nullptr;
-    constexpr int win_threads = 512;
+    int win_threads = 512;
     if (use_win) {
+        // many replicas: four CTAs of 256 threads an SM instead of two of 512 keep more windows in flight between
+        // the barriers (24 jobs, about 900 replicas: 720 -> 674 us); with fewer a window takes longer than it gains (131,072
+        // sites x 256, an earlier state of the kernel: 119 us with 512 threads, 136 with 256)
+        int dev = 0, n_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+        if (total >= 3 * n_sm) win_threads = 256;
         for (int j = 0; j < n_jobs; ++j) {
             const WinTab &w = hs[j]->win_host;
             smem = std::max(smem, WinLayout::make(w.n_ent, w.n_blk, hs[j]->n_cols).total);
