@@ -9,7 +9,7 @@ the whole job is 40 such steps.  Proposals come from the device Philox stream.
   value     swap attempts/s with the state resident in HBM, CUDA events around each chunk on its stream,
             L2 flushed (256 MB write) between timed chunks outside the events
   e2e       the same chunks through nce_ce_run_chunk_host: pinned host buffers in and out every chunk
-  roofline  dominant kernel ce_bin_chunk_kernel (sign-parity form); algorithmic bytes per attempt = 14,996 B
+  roofline  dominant kernel ce_win_chunk_kernel (windowed sign-parity form); algorithmic bytes per attempt = 14,996 B
             of int8 member-occupancy reads (2 x 7,498 member slots of the rows of both sites)
   cpu_baseline  the oracle's C restatement on the host cores (bounded sample, all threads)
   side lines  nce (configuration 1, float32), nce_tcgen05_split / nce_tcgen05_bf16 (the same on tcgen05
@@ -42,8 +42,8 @@ B_GATHER = 14_996                     # bytes of member occupancy per attempt, c
 # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from one ncu capture of the headline kernel,
 # keyed by (path, L, R, steps per chunk): profiles/ holds the capture (a 1000-step chunk; the tables and occupancy
 # are read once per launch, so the figure does not grow with the steps)
-TRAFFIC = {(2, 8, 32, 5000): 166_912}
-SMEM_PIPE = {(2, 8, 32, 5000): 0.178}       # the same capture's shared-memory wavefronts, fraction of the pipe's peak
+TRAFFIC = {(2, 8, 32, 5000): 159_744}
+SMEM_PIPE = {(2, 8, 32, 5000): 0.040}       # the same capture's shared-memory wavefronts, fraction of the pipe's peak
 
 
 def parse():
@@ -761,12 +761,12 @@ def main():
     ms_chunk = float(np.mean(per_ms))
     achieved = R * T * B_GATHER / (ms_chunk / 1e3) / 1e9
     # DRAM bytes per launch from one ncu capture of this workload (dram__bytes_read.sum + dram__bytes_write.sum of
-    # ce_bin_chunk_kernel, 2,048 sites, R = 32, 16 warps x 4 CTAs): the tables and occupancies live in shared memory;
+    # ce_win_chunk_kernel, 2,048 sites, R = 32): the tables live in shared memory, the occupancies in the L1 and L2;
     # the same capture's shared-memory pipe use (l1tex__data_pipe_lsu_wavefronts_mem_shared.sum.pct_of_peak_sustained
     # _elapsed), the on-chip roofline that the gathered bytes actually meet
     traffic = TRAFFIC.get((args.path, args.L, args.R, T))
     roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "traffic": traffic,
-            "kernel": {1: "ce_pt_chunk_kernel", 3: "ce_lf_chunk_kernel"}.get(args.path, "ce_bin_chunk_kernel"),
+            "kernel": {1: "ce_pt_chunk_kernel", 3: "ce_lf_chunk_kernel"}.get(args.path, "ce_win_chunk_kernel"),
             "peak_source": src,
             "algorithmic_bytes_per_launch": R * T * B_GATHER,
             "shared_pipe_frac_ncu": SMEM_PIPE.get((args.path, args.L, args.R, T))}
@@ -797,7 +797,7 @@ def main():
                 "warmup": args.warmup, "ms_per_step": ms_chunk, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": value / H100_PUBLISHED if (args.L == 8 and args.R == 32) else None,
                 "dtype": "f64" if args.precision == 64 else "f32", "data": "synthetic (seeded lattice, random-normal ECIs)",
-                "config": workload_config(args, gce), "clocks": clocks, "e2e": e2e, "gpu_launches": 2 * args.steps,
+                "config": workload_config(args, gce), "clocks": clocks, "e2e": e2e, "gpu_launches": args.steps,
                 "roofline": roof, "cpu_baseline": cpu, "nce": nce_line, "nce_tcgen05_split": nce_tc_line, "nce_tcgen05_bf16": nce_bf16_line, "nce_shipped_model": nce_shipped_line, "batch": batch_line, "serve": serve_line,
                 "large_ce": large_ce_line, "large_nce": large_nce_line,
                 "launch": {"warps_per_cta": args.warps, "ctas_per_replica": args.cluster,
