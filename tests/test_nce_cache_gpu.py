@@ -30,3 +30,30 @@ def test_batch_of_caches_equals_single(cuda, L, width, mma):
     # per-site energies: 1e-4 eV, the bound of the float32 and split forms; 2e-2 for plain bf16 operands
     assert np.abs(a.e[0].cpu().numpy() - np.asarray(c["e"])).max() < (2e-2 if mma == 2 else 1e-4)
     m.check_errors()
+
+
+@pytest.mark.parametrize("mma", [2, 4])
+def test_layer0_buffer_aligned_to_eight_bytes(cuda, mma):
+    """24 layer-0 channels (rows a multiple of four floats) in a buffer that starts between two 16-byte boundaries: caches and
+    steps equal those of an aligned buffer."""
+    torch = cuda
+    from neuralce_gb300.io import Z_OF, fcc_conventional
+    from neuralce_gb300.nce import NCEModel, NCEState, synthetic_model
+    from neuralce_gb300.workloads import A_FCC, cluster_space, random_occupancy
+    cs = cluster_space((7.5, 6.0, 4.2))
+    assert (len(cs.orbits) + 1) % 4 == 0
+    s = fcc_conventional(A_FCC, (4, 4, 4))
+    s.numbers = np.full(len(s), Z_OF["Ni"], np.int64)
+    P = synthetic_model(len(cs.orbits) + 1, 2, 32, 1, 1)
+    m = NCEModel(cs, s, P, shell_edges=(0.0, 3.3), act="silu", pool="sum", mma=mma)
+    sig = random_occupancy(len(s), 0.5, 2, 3)
+    a, b = NCEState(m, sig, np.full(2, 5.0)), NCEState(m, sig, np.full(2, 5.0))
+    buf = torch.zeros(b.h0.numel() + 2, dtype=torch.float32, device="cuda")
+    b.h0 = buf[2:].view(b.h0.shape)
+    assert b.h0.data_ptr() % 16 == 8
+    for st in (a, b):
+        st.full_cache()
+        st.run_chunk(12, 0, seed=4)
+    torch.cuda.synchronize()
+    for f in ("sigma", "h0", "hmid", "e", "E", "n_acc"):
+        assert torch.equal(getattr(a, f), getattr(b, f)), f
