@@ -25,6 +25,7 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 
+#include "ce_window_steps.cuh"
 #include "common.cuh"
 
 namespace cg = cooperative_groups;

@@ -20,7 +20,6 @@
 // exact fixed-point sum (float64) or the same float32 sum in the same order.
 
 constexpr int kWinRows = 7;              // rows a lane: 7 = the most that three adder words hold
-constexpr int kWinRing = 128;            // proposals in flight (a window reaches 32 steps ahead, drawn 64 ahead)
 constexpr int kWinSwaps = 16;            // swaps evaluated at once: two sites each fill the 32 bits of a word
 constexpr int kWinBatch = 9;             // neighbourhood entries a warp loads at once (141 entries on 16 warps: all)
 constexpr int kWinSegs = 4;               // column segments of a row block
@@ -95,7 +94,7 @@ __device__ __forceinline__ int win_entry(const CEJob &jb, const WinTab &wt, cons
 __device__ __forceinline__ void win_propose(const CEJob &jb, const WinTab &wt, const WinRing &ring, int64_t g0, int32_t s, int32_t t) {
     LfProp P;
     lf_propose(jb, g0, s, t, P);
-    const int i = s & (kWinRing - 1);
+    const int i = win_slot(s, 0);
     const int4 a = make_int4(P.ka[0], P.ka[1], P.ka[2], (int32_t)P.ia), b = make_int4(P.kb[0], P.kb[1], P.kb[2], (int32_t)P.ib);
     ring.a[i] = a; ring.b[i] = b;
     ring.u[i] = jb.prop_a ? (unsigned long long)__double_as_longlong(P.uh) : (unsigned long long)P.um;
@@ -190,11 +189,12 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
     const float scale_f = ldexpf(1.0f, -jb.fix_shift);
     const float tol_near = 1e-6f + 1.001f * beta_f * ((float)jb.near_eV + (FIX ? 4.0f * scale_f : 0.0f));
     const int32_t si = jb.E_samples && jb.sample_interval <= T ? (int32_t)jb.sample_interval : 0;
-    int32_t s_next = si;                                     // the next step to sample (1-based)
+    int32_t left = si;                                       // steps from the window's start to the next sample
     const double E0 = jb.E[r];
     double E = E0, Emin = jb.E_min_rep[r];                  // float32: carried energy and running minimum (warp 1)
     long long dsum = 0, dmin = 0;                            // float64: the chunk's energy change; this lane's minimum of it
-    int32_t nacc = 0, nnear = 0, drawn = 96, s_cur = 0, score = 0;
+    int32_t nacc = 0, nnear = 0, s_cur = 0, score = 0;
+    uint32_t drawn = 96;
     for (int q = tid; q < min(96, T); q += nt) win_propose(jb, wt, ring, g0, q, t);
     // this lane's columns (lane, lane + 32) of the dE sum; further columns, if any, are read where they are used
     const int c0 = lane, c1 = lane + 32;
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
     // warp 0: the window that starts at step s_cur, on the present occupancy, into X (X.step of the other parity)
     auto list_window = [&]() {
         const int avail = min(32, T - s_cur);
-        const int i = (s_cur + lane) & (kWinRing - 1);
+        const int i = win_slot(s_cur, lane);
         int sa = 0, sb = 0, known = 0, del = 0;
         int4 a = make_int4(0, 0, 0, 0), b = a;
         if (lane < avail) {
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
                     for (int n = nb; n >= 0 && (n = __ldg(wt.alias + n)) >= 0;) atomicXor(&words[n], 1u << lane);
                 }
             }
-            const int i = (s_w + lane) & (kWinRing - 1);
+            const int i = win_slot(s_w, lane);
             bool eq = false;
             if (lane > q && lane < n_w) {
                 const int pa = ring.a[i].w, pb = ring.b[i].w;
@@ -343,11 +343,11 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
                     if (sg[g].x) atomicAdd(&cnt[sg[g].y + lane], __popc(t1 & sg[g].x) + 2 * __popc(t2 & sg[g].x) + 4 * __popc(t4 & sg[g].x));
             }
         }
-        if (warp == nw - 1 && drawn < T && drawn < s_w + 96 && drawn + lane < T) {
-            win_propose(jb, wt, ring, g0, drawn + lane, t);
-            X.known[(drawn + lane) & (kWinRing - 1)] = 0;
+        if (warp == nw - 1 && win_draws(drawn, s_w) && win_in_chunk(drawn, lane, T)) {
+            win_propose(jb, wt, ring, g0, (int32_t)drawn + lane, t);
+            X.known[win_slot((int32_t)drawn, lane)] = 0;
         }
-        if (drawn < s_w + 96) drawn += 32;
+        if (win_draws(drawn, s_w)) drawn += 32;
         __syncthreads();
         if (nv > 0) {
             // 3. dE of each swap and its decision; what a swap accepted against its prediction changes
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
             for (int v = warp; v < kWinSwaps; v += nw) {
                 int32_t *ca = cnt + 2 * v, *cb = ca + 1;
                 if (v < nv) {
-                    const int i = (s_w + step[v]) & (kWinRing - 1);
+                    const int i = win_slot(s_w, step[v]);
                     const int sgn = X.spa[v] ? -1 : 1;
                     const unsigned long long u = ring.u[i];
                     const float lnu = ring.lnu[i];
@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
                     const int sa = X.spa[lane >> 1];
                     gsig[X.site[lane].w] = (int8_t)((lane & 1) ? sa : 1 - sa);
                 }
-                if (lane < nv && q >= limit) X.known[(s_w + q) & (kWinRing - 1)] = (flags & 1) ? 1 : 2;
+                if (lane < nv && q >= limit) X.known[win_slot(s_w, q)] = (flags & 1) ? 1 : 2;
                 const unsigned decided = __ballot_sync(0xffffffffu, lane < nv && q < limit);
                 score = max(-64, min(64, score + 2 * __popc(acc) - __popc(decided)));
                 s_cur = s_w + limit;
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
                 if (track)                                      // tracked sums: each changed row moves its column by +-2
                     for (unsigned m = acc; m; m &= m - 1)
                         for (int c = lane; c < n_cols; c += 32) dcv[c] += 2 * (int)nsw[(__ffs(m) - 1) * n_cols + c];
-                const bool sample = si > 0 && s_next <= s_w + limit;
+                const bool sample = si > 0 && left <= limit;
                 long long pre = dsum; double Epre = E;          // energy after this lane's step (when sampled)
                 if (FIX) {
                     long long run = mine ? part : 0;            // inclusive sum over the accepted swaps
@@ -451,12 +451,9 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
                         if (__shfl_sync(0xffffffffu, q, v) <= lane) Epre = E;
                     }
                 }
-                if (sample) {
-                    const int s1 = s_w + lane + 1;
-                    if (lane < limit && s1 >= s_next && (s1 - s_next) % si == 0)
-                        jb.E_samples[(int64_t)(s1 / si - 1) * jb.R + t] = FIX ? E0 + (double)pre * fscale : Epre;
-                    s_next += (s_w + limit - s_next) / si * si + si;
-                }
+                if (sample && win_samples(left, si, lane, limit))
+                    jb.E_samples[(int64_t)((s_w + lane + 1) / si - 1) * jb.R + t] = FIX ? E0 + (double)pre * fscale : Epre;
+                if (si > 0) left = win_left(left, si, limit);
             }
         }
     }
