@@ -7,7 +7,7 @@
 //                       every reverse row of both sites with warp-parallel products of point functions,
 //                       reduces dE with warp shuffles, applies the Metropolis rule and writes the two sites.
 //                       Row tables are staged in shared memory once per chunk.
-//   ce_exchange_kernel  chunk-end replica exchange of temperature slots (one CTA per job).
+//   ce_exchange_kernel  chunk-end replica exchange of temperature slots (one warp per job).
 //   ce_energy_kernel    full energy: cells x template rows, per-block float64 partials, fixed-order sum.
 //   ce_delta_kernel     batched swap dE queries through the same block routine as the chunk kernel.
 #include <cuda_runtime.h>
@@ -25,6 +25,7 @@
 #include <cooperative_groups.h>
 #include <type_traits>
 
+#include "ce_exchange.cuh"
 #include "ce_window_steps.cuh"
 #include "common.cuh"
 
@@ -273,54 +274,6 @@ __device__ __forceinline__ void propose(const CEJob &jb, int64_t g, int32_t t, i
     ia = (int64_t)draw_index(x.x, nc) * jb.nB + __ldg(jb.act_b + grp * jb.max_gb + ba);
     ib = (int64_t)draw_index(x.y, nc) * jb.nB + __ldg(jb.act_b + grp * jb.max_gb + bb);
     u = draw_u01(x.z, x.w);
-}
-
-// Chunk end, called by one whole warp of each replica (the cluster's first CTA) once its outputs are written: the last
-// replica of the job to arrive performs the job's slot exchange -- the rule, random counters and sample rewrite of
-// ce_exchange_kernel, with the pairs swapped in place -- advances the device step counter and re-arms the counter.
-// No thread waits for another, so the chunk kernel never depends on its CTAs running at the same time.  The pairs of an
-// exchange are disjoint, so a lane takes a pair: one thread walking them spent about 1 us a pair on dependent loads and
-// a float64 logarithm at the end of every chunk (256 replicas of 131,072 sites, chunks of 300 steps: 1,462 -> 1,196 us; 16 of 256 sites, 10 steps: 77 -> 63 us).
-__device__ void fused_chunk_end(const CEJob &jb, int64_t g0, int lane) {
-    int last = 0;
-    if (lane == 0) {
-        __threadfence();                                  // this replica's energy is visible before it is counted
-        last = atomicAdd(jb.ex_sync, 1) == jb.R - 1;
-    }
-    if (!__shfl_sync(0xffffffffu, last, 0)) return;
-    __threadfence();
-    const int R = jb.R;
-    const int64_t g_end = g0 + jb.n_steps;
-    if (lane == 0 && jb.step_dev) *const_cast<int64_t *>(jb.step_dev) = g_end;   // every CTA of the job has read it by now
-    if ((jb.ex_flags & 1) && R > 1) {
-        const uint32_t k0 = (uint32_t)jb.seed, k1 = (uint32_t)(jb.seed >> 32);
-        const uint32_t c0 = (uint32_t)g_end, c1 = (uint32_t)((uint64_t)g_end >> 32);
-        const uint32_t cq = 0xFFFFFFFFu;                   // round 0 of the exchange counters
-        const int parity = jb.ex_u ? ((jb.ex_flags >> 1) & 1) : (int)(philox4x32(c0, c1, cq, 0u, k0, k1).x & 1u);
-        int32_t *ros = jb.rep_of_slot;
-        int nswap = 0;
-        for (int k = lane; 2 * k < R - 1; k += 32) {
-            const int a = 2 * k + parity, b = a + 1;
-            if (b >= R || jb.ladder_id[a] != jb.ladder_id[b]) continue;
-            const int32_t ra = __ldcg(ros + a), rb = __ldcg(ros + b);
-            const double Ea = __ldcg(jb.E + ra), Eb = __ldcg(jb.E + rb);
-            const double log_acc = ((double)jb.beta_slot[b] - (double)jb.beta_slot[a]) * (Eb - Ea);
-            double u;
-            if (jb.ex_u) u = jb.ex_u[k];
-            else { const u32x4 w = philox4x32(c0, c1, cq - 1u, (uint32_t)k, k0, k1); u = draw_u01(w.x, w.y); }
-            if (log(u) < log_acc) { ros[a] = rb; ros[b] = ra; ++nswap; }
-        }
-        nswap = __reduce_add_sync(0xffffffffu, nswap);
-        if (lane == 0) *jb.n_ex += nswap;
-        const bool rewrite = jb.E_samples && jb.n_steps > 0 && jb.n_steps % jb.sample_interval == 0;
-        const int64_t row = rewrite ? jb.n_steps / jb.sample_interval - 1 : 0;
-        for (int q = lane; q < R; q += 32) {
-            const int32_t rq = __ldcg(ros + q);
-            jb.slot_of_rep[rq] = q;
-            if (rewrite) jb.E_samples[row * R + q] = __ldcg(jb.E + rq);
-        }
-    }
-    if (lane == 0) *jb.ex_sync = 0;
 }
 
 template <typename Real, int MO>
@@ -1466,7 +1419,7 @@ struct CEExJob {
 };
 struct CEExBatch { int32_t n_jobs; CEExJob job[kMaxJobs]; };
 
-// (one warp a job: a lane a pair of slots, as in fused_chunk_end; the pairs of a round are disjoint)
+// (one warp a job)
 __global__ void ce_exchange_kernel(const __grid_constant__ CEExBatch bt) {
     const int j = blockIdx.x, lane = threadIdx.x;
     if (j >= bt.n_jobs || lane >= 32) return;
@@ -1475,35 +1428,12 @@ __global__ void ce_exchange_kernel(const __grid_constant__ CEExBatch bt) {
     __syncwarp();
     if (lane == 0 && x.step_dev) *x.step_dev = g_end;      // the chunk kernel has finished reading it (stream order)
     if (!x.do_exchange || x.R < 2) return;
-    const int R = x.R;
-    const uint32_t k0 = (uint32_t)x.seed, k1 = (uint32_t)(x.seed >> 32);
-    const uint32_t c0 = (uint32_t)g_end, c1 = (uint32_t)((uint64_t)g_end >> 32);
-    const int npair = R / 2;                 // ceil((R-1)/2)
-    int nswap = 0;
-    for (int q = 0; q < max(x.rounds, 1); ++q) {
-        const uint32_t cq = 0xFFFFFFFFu - 2u * (uint32_t)q;
-        const int parity = x.ex_u ? ((x.parity >> q) & 1) : (int)(philox4x32(c0, c1, cq, 0u, k0, k1).x & 1u);
-        for (int k = lane; 2 * k < R - 1; k += 32) {
-            const int a = 2 * k + parity, b = a + 1;
-            if (b >= R) continue;
-            if (x.ladder_id[a] != x.ladder_id[b]) continue;
-            const int32_t ra = x.rep_of_slot[a], rb = x.rep_of_slot[b];
-            const double Ea = x.E[ra] * x.E_scale, Eb = x.E[rb] * x.E_scale;
-            const double log_acc = ((double)x.beta_slot[b] - (double)x.beta_slot[a]) * (Eb - Ea);
-            double u;
-            if (x.ex_u) u = x.ex_u[(size_t)q * npair + k];
-            else { u32x4 w = philox4x32(c0, c1, cq - 1u, (uint32_t)k, k0, k1); u = draw_u01(w.x, w.y); }
-            if (log(u) < log_acc) { x.rep_of_slot[a] = rb; x.rep_of_slot[b] = ra; ++nswap; }
-        }
-        __syncwarp();                        // the next round pairs the slots as this one left them
-    }
-    nswap = __reduce_add_sync(0xffffffffu, nswap);
-    if (lane == 0) *x.n_ex += nswap;
-    for (int t = lane; t < R; t += 32) {
-        const int32_t rt = x.rep_of_slot[t];
-        x.slot_of_rep[rt] = t;
-        if (x.E_samples && x.last_row >= 0) x.E_samples[x.last_row * R + t] = x.E[rt];
-    }
+    ExArgs a;
+    a.R = x.R; a.E = x.E; a.E_scale = x.E_scale; a.beta_slot = x.beta_slot; a.rep_of_slot = x.rep_of_slot;
+    a.slot_of_rep = x.slot_of_rep; a.ladder_id = x.ladder_id; a.n_ex = x.n_ex; a.seed = x.seed; a.g_end = g_end;
+    a.ex_u = x.ex_u; a.parity = x.parity; a.rounds = max(x.rounds, 1);
+    a.E_samples = x.last_row >= 0 ? x.E_samples : nullptr; a.row = x.last_row;
+    exchange_warp(a, lane);
 }
 
 // full energy: grid (blocks_per_rep, R); per-block float64 partial -> partial[r * nblk + bx]
