@@ -98,7 +98,8 @@ __device__ __forceinline__ void win_propose(const CEJob &jb, const WinTab &wt, c
     const int4 a = make_int4(P.ka[0], P.ka[1], P.ka[2], (int32_t)P.ia), b = make_int4(P.kb[0], P.kb[1], P.kb[2], (int32_t)P.ib);
     ring.a[i] = a; ring.b[i] = b;
     ring.u[i] = jb.prop_a ? (unsigned long long)__double_as_longlong(P.uh) : (unsigned long long)P.um;
-    ring.lnu[i] = P.lnu;
+    // (a host uniform below 0 or NaN has no logarithm: the float64 rule takes it, and rejects)
+    ring.lnu[i] = jb.prop_a && !(P.uh >= 0.0) ? nanf("") : P.lnu;
     ring.del[i] = win_disp(jb, wt, a, b);
 }
 
@@ -109,7 +110,8 @@ __device__ __noinline__ double win_log(bool host, unsigned long long u) {
 
 // Metropolis decision and near-threshold flag of dE.  float32 settles a swap whose |beta dE + ln u| exceeds its own error
 // (below 1e-6 + 1e-6 (|beta dE| + |ln u|)) and the near band (tol_near); the others (about one in 10^5) take the exact
-// rule: the fixed-point threshold ceil(-ln u / beta 2^S) (float64) or ln u < -beta dE in float64 (float32).
+// rule: the fixed-point threshold ceil(-ln u / beta 2^S) (float64) or ln u < -beta dE in float64 (float32).  So does every
+// swap at a beta below 0 or NaN, where the fixed-point rule has no such threshold and the band no width.
 __device__ __forceinline__ int win_decide_fix(const CEJob &jb, long long part, unsigned long long u, float lnu, float beta_f,
                                               float scale_f, float tol_near) {
     const float bd = beta_f * ((float)part * scale_f), y = bd + lnu;
@@ -187,7 +189,8 @@ __global__ void __launch_bounds__(512, MINB) ce_win_chunk_kernel(const __grid_co
     const int64_t g0 = jb.step_dev ? *jb.step_dev : jb.step0;
     const double fscale = ldexp(1.0, -jb.fix_shift);
     const float scale_f = ldexpf(1.0f, -jb.fix_shift);
-    const float tol_near = 1e-6f + 1.001f * beta_f * ((float)jb.near_eV + (FIX ? 4.0f * scale_f : 0.0f));
+    // (beta below 0 or NaN: nothing is settled in float32)
+    const float tol_near = beta_f >= 0.0f ? 1e-6f + 1.001f * beta_f * ((float)jb.near_eV + (FIX ? 4.0f * scale_f : 0.0f)) : HUGE_VALF;
     const int32_t si = jb.E_samples && jb.sample_interval <= T ? (int32_t)jb.sample_interval : 0;
     int32_t left = si;                                       // steps from the window's start to the next sample
     const double E0 = jb.E[r];
