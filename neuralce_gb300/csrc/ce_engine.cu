@@ -1329,6 +1329,68 @@ __global__ void __launch_bounds__(kEnThreads) ce_energy_bits_kernel(const uint32
         if (ccnt[c]) atomicAdd(cv + (int64_t)r * n_cols + c, ccnt[c]);
 }
 
+// The same sums for sets whose distinct member offsets do not fit a thread's column of shared memory (neighbourhoods of
+// more than about 1,400 sites): every member's word is fetched for every row, about 22 instructions a member, bound by the
+// issue rate (1,048,576 sites x 64 of the 8 / 6 / 5 A set: 7.34 ms against 1.16 above).
+// grid (item blocks x row slices, nB, R): threads over the (k0, k1, 32-anchor word) items of anchor basis
+// blockIdx.y, replica blockIdx.z; a small cell's rows are split into slices over more blocks.  Every lane of a
+// warp walks the same rows (lanes past the last item count nothing).
+__global__ void __launch_bounds__(256) ce_energy_rows_kernel(const uint32_t *__restrict__ planes, int32_t P, int32_t d0, int32_t d1,
+                                                              int32_t d2, int32_t W2, const uint32_t *__restrict__ brows,
+                                                              const int4 *__restrict__ bmem, const int32_t *__restrict__ brow_off,
+                                                              const int32_t *__restrict__ brow_n, int32_t n_cols, int32_t slices,
+                                                              unsigned long long *__restrict__ cv) {
+    extern __shared__ unsigned long long ccnt[];
+    const int b = blockIdx.y, r = blockIdx.z, lane = threadIdx.x & 31;
+    const int slice = (int)(blockIdx.x % (unsigned)slices), iblk = (int)(blockIdx.x / (unsigned)slices);
+    const int iblocks = (int)(gridDim.x / (unsigned)slices);
+    for (int c = threadIdx.x; c < n_cols; c += blockDim.x) ccnt[c] = 0ull;
+    __syncthreads();
+    const int Wn = (d2 + 31) >> 5;
+    const int64_t items = (int64_t)d0 * d1 * Wn;
+    const uint32_t *pr = planes + (int64_t)r * P * d0 * d1 * W2;
+    const int nall = brow_n[b];
+    const int q0 = (int)((int64_t)nall * slice / slices), q1 = (int)((int64_t)nall * (slice + 1) / slices);
+    const uint32_t *rows = brows + brow_off[b];
+    auto flush = [&](int col, int acc) {
+        const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)acc);
+        if (lane == 0 && sum) atomicAdd(&ccnt[col], (unsigned long long)(long long)sum);
+    };
+    for (int64_t base = (int64_t)iblk * blockDim.x; base < items; base += (int64_t)iblocks * blockDim.x) {
+        const int64_t it = base + threadIdx.x;
+        const bool live = it < items;
+        const int64_t itc = live ? it : 0;
+        const int w = (int)(itc % Wn);
+        const int64_t kk = itc / Wn;
+        const int k1 = (int)(kk % d1), k0 = (int)(kk / d1);
+        const int nv = live ? min(32, d2 - 32 * w) : 0;
+        const uint32_t mask = nv >= 32 ? 0xffffffffu : ((1u << nv) - 1u);
+        int col = -1, acc = 0;
+        for (int q = q0; q < q1; ++q) {
+            const uint32_t rd = __ldg(rows + q);
+            const int c = (int)(rd & 0xffu), nm = (int)((rd >> 8) & 0xfu), st = (int)(rd >> 12);
+            if (c != col) {
+                if (col >= 0) flush(col, acc);
+                col = c; acc = 0;
+            }
+            uint32_t par = 0;
+            for (int m = 0; m < nm; ++m) {
+                const int4 e = __ldg(bmem + st + m);           // (plane, uo0, uo1, uo2)
+                int a0 = k0 + e.y; a0 -= a0 >= d0 ? d0 : 0;
+                int a1 = k1 + e.z; a1 -= a1 >= d1 ? d1 : 0;
+                const int pos = 32 * w + e.w;
+                const uint32_t *row = pr + (((int64_t)e.x * d0 + a0) * d1 + a1) * W2 + (pos >> 5);
+                par ^= __funnelshift_r(__ldg(row), __ldg(row + 1), (unsigned)(pos & 31));
+            }
+            acc += nv - 2 * __popc(par & mask);
+        }
+        if (col >= 0) flush(col, acc);
+    }
+    __syncthreads();
+    for (int c = threadIdx.x; c < n_cols; c += blockDim.x)
+        if (ccnt[c]) atomicAdd(cv + (int64_t)r * n_cols + c, ccnt[c]);
+}
+
 // Local fields of every site of R configurations, bit-sliced like the full energy: a thread takes 32 consecutive
 // sites along k2 of one basis and, for every reverse row of that basis (every cluster instance containing the
 // site), XORs the members' shifted plane words (bit j: the parity of site j's product); odd parities are counted
@@ -1546,6 +1608,10 @@ struct nce_ce_model {
     // point-function column of each plane
     uint4 *bwords = nullptr; int32_t *bword_off = nullptr, *bgrp_off = nullptr; uint32_t *brows[2] = {nullptr, nullptr}, *bgrp = nullptr;
     int32_t bw_max = 0, bw_oth = 3;
+    // the same for sets with more offsets or members than that kernel takes (bgrp null): rows anchored at a site (col | members
+    // << 8 | first member << 12) per basis, members (plane, uo0, uo1, uo2)
+    uint32_t *erows = nullptr; int4 *emem = nullptr; int32_t *erow_off = nullptr, *erow_n = nullptr;
+    bool has_counts() const { return binary && (bgrp || erows); }
     bool plane32 = false; uint32_t plane_flip = 0;    // planes of one basis site with species 0 / 1 (ce_bitplane32_kernel)
     int32_t *plane_pfc = nullptr; int32_t n_planes = 0;
     double *ecol1 = nullptr;                 // eci of each column (full-energy kernel)
@@ -1579,7 +1645,7 @@ static int upload(T *&dst, const T *src, size_t n) {
 
 static int free_model(nce_ce_model *m) {
     void *ptrs[] = {m->loc, m->pfc, m->eci64, m->eci32, m->rv_len, m->nb_b, m->nb_uo, m->pf64, m->pf32, m->act_b,
-                    m->act_nb, m->grp_cum, m->T_b, m->T_uo, m->T_pfc, m->T_eci64, m->T_eci32, m->err, m->sbits, m->bix, m->rcol, m->ecol2_64, m->ecol2_32, m->ecol_fix, m->chunks, m->n_chunks, m->brows[0], m->brows[1], m->bwords, m->bword_off, m->bgrp_off, m->bgrp, m->plane_pfc, m->ecol1,
+                    m->act_nb, m->grp_cum, m->T_b, m->T_uo, m->T_pfc, m->T_eci64, m->T_eci32, m->err, m->sbits, m->bix, m->rcol, m->ecol2_64, m->ecol2_32, m->ecol_fix, m->chunks, m->n_chunks, m->brows[0], m->brows[1], m->bwords, m->bword_off, m->bgrp_off, m->bgrp, m->erows, m->emem, m->erow_off, m->erow_n, m->plane_pfc, m->ecol1,
                     m->staging_base, m->lf_off, m->lf_idx, m->lf_box, m->frows, m->fmem, m->frow_off, m->frow_n,
                     m->win, m->win_ent, m->win_desc, m->win_seg, m->win_nbr, m->win_alias, m->win_csign};
     for (void *p : ptrs) if (p) cudaFree(p);
@@ -2004,7 +2070,7 @@ static int launch_delta(const CEJob &jb, int mo, int n, const int32_t *rep, cons
 namespace nce {
 int ce_model_dims(nce_ce_handle h, int64_t *N, int32_t *n_cols, int32_t *mo, int32_t *binary) {
     NCE_CHECK(h, "null CE handle");
-    *N = h->N; *n_cols = h->n_cols; *mo = h->mo; *binary = (h->binary && h->bgrp) ? 1 : 0;
+    *N = h->N; *n_cols = h->n_cols; *mo = h->mo; *binary = h->has_counts() ? 1 : 0;
     return NCE_OK;
 }
 }  // namespace nce
@@ -2386,7 +2452,6 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                 // change sign: (anchor basis, column) -> members beside the anchor
                 typedef std::array<int32_t, 4> Mem;              // plane * nB + basis, uo0, uo1, uo2
                 std::vector<std::vector<std::vector<std::vector<Mem>>>> inst((size_t)t->nB, std::vector<std::vector<std::vector<Mem>>>((size_t)t->n_cols));
-                std::vector<char> has_own((size_t)t->nB, 0);
                 int oth = 0;
                 for (int b = 0; b < t->nB; ++b)
                     for (int q = 0; q < t->Rv_len[b]; ++q) {
@@ -2421,17 +2486,19 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                         oth = std::max(oth, (int)rel.size() - 1);
                     }
                 m->bw_oth = oth <= 3 ? 3 : 7;
+                // (the kernel forms plane rows in 32 bits)
+                bool by_words = (int64_t)ppfc.size() * t->nB * t->d[0] * t->d[1] < (1ll << 31);
                 for (int b = 0; b < t->nB; ++b) {
                     std::map<Mem, int> at;
                     for (const auto &col : inst[b]) for (const auto &rel : col) if (!rel.empty()) at[rel[0]] = 0;
                     // several point-function columns on one basis site: a row anchored on another than the first XORs the first
                     // away and its own in (two more words)
                     if (at.size() > 1) m->bw_oth = 7;
-                    if (oth + (at.size() > 1 ? 2 : 0) > 7) bin = false;
+                    if (oth + (at.size() > 1 ? 2 : 0) > 7) by_words = false;
                 }
                 std::vector<uint4> words; std::vector<int32_t> word_off(1, 0), grp_off(1, 0);
                 std::vector<uint32_t> idx, info;                 // (groups, 3, bw_oth + 1) word indices; column | rows << 16
-                for (int b = 0; b < t->nB && bin; ++b) {
+                for (int b = 0; b < t->nB && by_words; ++b) {
                     std::map<Mem, int> at;                       // the anchor's own words first, the others by row
                     for (const auto &col : inst[b]) for (const auto &rel : col) if (!rel.empty()) at[rel[0]] = 0;
                     std::vector<Mem> order;
@@ -2469,8 +2536,32 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                     grp_off.push_back((int32_t)info.size());
                 }
                 // a thread's column of words must fit shared memory with one word a thread at least
-                if (m->bw_max > 700) bin = false;
-                if (bin && !ppfc.empty()) {
+                by_words = by_words && m->bw_max <= 700;
+                std::vector<uint32_t> rows; std::vector<int4> mem; std::vector<int32_t> roff(t->nB), rn(t->nB);
+                for (int b = 0; b < t->nB && !by_words; ++b) {   // otherwise rows as listed, with all their members
+                    roff[b] = (int32_t)rows.size();
+                    for (int q = 0; q < t->Rv_len[b]; ++q) {
+                        if (t->Rv_slot[(size_t)b * t->J + q] != 0) continue;
+                        const uint32_t start = (uint32_t)mem.size();
+                        for (int k = 0; k < t->mo; ++k) {
+                            const size_t e = ((size_t)b * t->J + q) * t->mo + k;
+                            const int pl = pmap[t->Rv_pfc[e]];
+                            if (pl < 0) continue;                          // constant point function (padded member)
+                            const size_t nb = (size_t)b * t->n_nbr + t->Rv_loc[e];
+                            mem.push_back(make_int4(pl * t->nB + t->nb_b[nb], t->nb_uo[3 * nb], t->nb_uo[3 * nb + 1], t->nb_uo[3 * nb + 2]));
+                        }
+                        if (start >= (1u << 20)) { bin = false; break; }
+                        rows.push_back((uint32_t)t->Rv_col[(size_t)b * t->J + q] | ((uint32_t)(mem.size() - start) << 8) | (start << 12));
+                    }
+                    rn[b] = (int32_t)rows.size() - roff[b];
+                }
+                if (bin && !ppfc.empty() && !by_words) {
+                    if (!rc) rc = upload(m->erows, rows.data(), rows.size());
+                    if (!rc) rc = upload(m->emem, mem.data(), mem.size());
+                    if (!rc) rc = upload(m->erow_off, roff.data(), roff.size());
+                    if (!rc) rc = upload(m->erow_n, rn.data(), rn.size());
+                }
+                if (by_words && !ppfc.empty()) {
                     for (int k = 0; k < 2; ++k) {                // as shared-memory word offsets: one and two words a thread
                         std::vector<uint32_t> o(idx);
                         for (auto &v : o) v *= kEnThreads << k;
@@ -2480,6 +2571,8 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                     if (!rc) rc = upload(m->bword_off, word_off.data(), word_off.size());
                     if (!rc) rc = upload(m->bgrp_off, grp_off.data(), grp_off.size());
                     if (!rc) rc = upload(m->bgrp, info.data(), info.size());
+                }
+                if (bin && !ppfc.empty()) {
                     m->plane32 = t->nB == 1 && t->max_sp <= 2 && ppfc.size() == 1 && t->d[2] % 32 == 0;
                     m->plane_flip = sb[(size_t)ppfc[0] * 4] ? 0xffffffffu : 0u;
                     m->plane32 = m->plane32 && sb[(size_t)ppfc[0] * 4] != sb[(size_t)ppfc[0] * 4 + 1];
@@ -2488,7 +2581,7 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                     m->n_planes = (int32_t)ppfc.size();
                 }
             }
-            if (!rc && bin && m->bgrp && m->fix_shift > 0) rc = build_local_field_tables(m, t, sb);
+            if (!rc && bin && (m->bgrp || m->erows) && m->fix_shift > 0) rc = build_local_field_tables(m, t, sb);
             if (!rc && bin) rc = build_window_tables(m, t, sb);
             m->binary = !rc;
         }
@@ -2513,7 +2606,7 @@ int nce_ce_energy(nce_ce_handle h, const int8_t *sigma, int32_t R, int32_t preci
 
 int nce_ce_cluster_counts(nce_ce_handle h, const int8_t *sigma, int32_t R, int64_t *cv, void *stream) {
     NCE_CHECK(h && sigma && cv && R >= 1, "nce_ce_cluster_counts: bad argument");
-    NCE_CHECK(h->binary && h->bgrp, "nce_ce_cluster_counts: needs point functions in {-1, +1}");
+    NCE_CHECK(h->has_counts(), "nce_ce_cluster_counts: needs point functions in {-1, +1}");
     std::lock_guard<std::mutex> lk(h->mu);
     cudaStream_t s = (cudaStream_t)stream;
     NCE_CUDA(cudaMemsetAsync(cv, 0, sizeof(int64_t) * (size_t)R * h->n_cols, s));
@@ -2550,7 +2643,7 @@ static int launch_planes(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_
 // kernel only, zeroed by the caller); E may be null when only the sums are wanted
 static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t precision, double *E, int64_t *cv_out,
                        cudaStream_t s) {
-    if (h->binary && h->bgrp) {
+    if (h->has_counts()) {
         // sign-parity full energy, bit-sliced: planes of the configurations, exact column sums, float64 energy
         NCE_CHECK(R <= 65535, "energy: at most 65535 configurations per call");
         const int64_t d0 = h->d[0], d1 = h->d[1], d2 = h->d[2];
@@ -2571,6 +2664,13 @@ static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t 
         const int64_t items = d0 * d1 * ((d2 + 31) / 32);
         int nsm = 152;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
+        if (!h->bgrp) {                                          // (every slice of the rows over more blocks, as below)
+            const int64_t ib = std::min<int64_t>((items + 255) / 256, 8192), have = ib * h->nB * R;
+            const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(32, (4ll * nsm + have - 1) / have));
+            ce_energy_rows_kernel<<<dim3((unsigned)(ib * slices), h->nB, R), 256, sizeof(unsigned long long) * h->n_cols, s>>>(
+                (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->erows, h->emem, h->erow_off, h->erow_n,
+                h->n_cols, slices, (unsigned long long *)cv);
+        } else {
         // two words a thread where that still fills the SMs several times over (a row's descriptor and addresses serve both; four
         // left too few warps: no faster); small cells: one, and the rows split into slices so that the launch covers the SMs
         // (about 4 blocks per SM; every slice fetches the words again)
@@ -2587,6 +2687,7 @@ static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t 
         kern<<<dim3((unsigned)(ib * slices), h->nB, R), kEnThreads, sm, s>>>(
             (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->bwords, h->bword_off, h->brows[kw],
             h->bgrp_off, h->bgrp, h->n_cols, slices, h->bw_max, (unsigned long long *)cv);
+        }
         NCE_CUDA(cudaGetLastError());
         if (E) {
             ce_energy_counts_kernel<<<(R + 127) / 128, 128, 0, s>>>(cv, R, h->n_cols, h->ecol1, h->zerolet, E);
