@@ -1329,9 +1329,9 @@ __global__ void __launch_bounds__(kEnThreads) ce_energy_bits_kernel(const uint32
         if (ccnt[c]) atomicAdd(cv + (int64_t)r * n_cols + c, ccnt[c]);
 }
 
-// The same sums for sets whose distinct member offsets do not fit a thread's column of shared memory (neighbourhoods of
-// more than about 1,400 sites): every member's word is fetched for every row, about 22 instructions a member, bound by the
-// issue rate (1,048,576 sites x 64 of the 8 / 6 / 5 A set: 7.34 ms against 1.16 above).
+// The same sums with every member's word fetched for every row, about 22 instructions a member, bound by the issue rate
+// (1,048,576 sites x 64 of the 8 / 6 / 5 A set: 7.34 ms against 1.16 above): for sets whose distinct offsets do not fit a
+// thread's column of shared memory, and where words are shared by too few rows to pay (energy_impl).
 // grid (item blocks x row slices, nB, R): threads over the (k0, k1, 32-anchor word) items of anchor basis
 // blockIdx.y, replica blockIdx.z; a small cell's rows are split into slices over more blocks.  Every lane of a
 // warp walks the same rows (lanes past the last item count nothing).
@@ -1608,9 +1608,10 @@ struct nce_ce_model {
     // point-function column of each plane
     uint4 *bwords = nullptr; int32_t *bword_off = nullptr, *bgrp_off = nullptr; uint32_t *brows[2] = {nullptr, nullptr}, *bgrp = nullptr;
     int32_t bw_max = 0, bw_oth = 3;
-    // the same for sets with more offsets or members than that kernel takes (bgrp null): rows anchored at a site (col | members
-    // << 8 | first member << 12) per basis, members (plane, uo0, uo1, uo2)
+    // the same for the kernel that fetches every member (any set; the only one where bgrp is null): rows anchored at a site
+    // (col | members << 8 | first member << 12) per basis, members (plane, uo0, uo1, uo2)
     uint32_t *erows = nullptr; int4 *emem = nullptr; int32_t *erow_off = nullptr, *erow_n = nullptr;
+    int64_t e_words = 0, e_members = 0;      // distinct offsets and members of all rows, over the bases
     bool has_counts() const { return binary && (bgrp || erows); }
     bool plane32 = false; uint32_t plane_flip = 0;    // planes of one basis site with species 0 / 1 (ce_bitplane32_kernel)
     int32_t *plane_pfc = nullptr; int32_t n_planes = 0;
@@ -2538,7 +2539,8 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                 // a thread's column of words must fit shared memory with one word a thread at least
                 by_words = by_words && m->bw_max <= 700;
                 std::vector<uint32_t> rows; std::vector<int4> mem; std::vector<int32_t> roff(t->nB), rn(t->nB);
-                for (int b = 0; b < t->nB && !by_words; ++b) {   // otherwise rows as listed, with all their members
+                bool by_rows = true;
+                for (int b = 0; b < t->nB; ++b) {                // rows as listed, with all their members
                     roff[b] = (int32_t)rows.size();
                     for (int q = 0; q < t->Rv_len[b]; ++q) {
                         if (t->Rv_slot[(size_t)b * t->J + q] != 0) continue;
@@ -2550,12 +2552,14 @@ int nce_ce_create(const nce_ce_tables *t, nce_ce_handle *out) {
                             const size_t nb = (size_t)b * t->n_nbr + t->Rv_loc[e];
                             mem.push_back(make_int4(pl * t->nB + t->nb_b[nb], t->nb_uo[3 * nb], t->nb_uo[3 * nb + 1], t->nb_uo[3 * nb + 2]));
                         }
-                        if (start >= (1u << 20)) { bin = false; break; }
+                        if (start >= (1u << 20)) { by_rows = false; break; }
                         rows.push_back((uint32_t)t->Rv_col[(size_t)b * t->J + q] | ((uint32_t)(mem.size() - start) << 8) | (start << 12));
                     }
                     rn[b] = (int32_t)rows.size() - roff[b];
                 }
-                if (bin && !ppfc.empty() && !by_words) {
+                bin = bin && (by_words || by_rows);
+                m->e_words = (int64_t)words.size(); m->e_members = (int64_t)mem.size();
+                if (by_rows && !ppfc.empty()) {
                     if (!rc) rc = upload(m->erows, rows.data(), rows.size());
                     if (!rc) rc = upload(m->emem, mem.data(), mem.size());
                     if (!rc) rc = upload(m->erow_off, roff.data(), roff.size());
@@ -2664,23 +2668,35 @@ static int energy_impl(nce_ce_model *h, const int8_t *sigma, int32_t R, int32_t 
         const int64_t items = d0 * d1 * ((d2 + 31) / 32);
         int nsm = 152;
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-        if (!h->bgrp) {                                          // (every slice of the rows over more blocks, as below)
-            const int64_t ib = std::min<int64_t>((items + 255) / 256, 8192), have = ib * h->nB * R;
-            const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(32, (4ll * nsm + have - 1) / have));
-            ce_energy_rows_kernel<<<dim3((unsigned)(ib * slices), h->nB, R), 256, sizeof(unsigned long long) * h->n_cols, s>>>(
-                (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->erows, h->emem, h->erow_off, h->erow_n,
-                h->n_cols, slices, (unsigned long long *)cv);
-        } else {
         // two words a thread where that still fills the SMs several times over (a row's descriptor and addresses serve both; four
         // left too few warps: no faster); small cells: one, and the rows split into slices so that the launch covers the SMs
-        // (about 4 blocks per SM; every slice fetches the words again)
+        // (about 4 blocks per SM, or as many as fit one; every slice fetches the words again)
         const int kw = items * h->nB * R >= 16ll * nsm * kEnThreads * 2 &&
                        sizeof(uint32_t) * 2 * kEnThreads * (size_t)(h->bw_max + 1) <= 100 * 1024;
         const int per = kEnThreads << kw;
         const int64_t ib = std::min<int64_t>((items + per - 1) / per, 8192);
         const int64_t have = ib * h->nB * R;
-        const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(8, (4ll * nsm + have - 1) / have));
         const size_t sm = sizeof(uint32_t) * per * (size_t)(h->bw_max + 1) + sizeof(unsigned long long) * h->n_cols;
+        const int fit = (int)std::min<size_t>(4, (208 * 1024) / (sm + 1024));      // (some of an SM's memory left to the planes' lines)
+        const int slices = (int)std::max<int64_t>(1, std::min<int64_t>(8, fit >= 4 ? (4ll * nsm + have - 1) / have : fit * (int64_t)nsm / have));
+        // words pay where their fetches, once a slice, are fewer than the rows' members; where few blocks fit an SM to hide the
+        // fetches' latency, several times fewer.  Kernel us, every member / words (words of up to 8 slices):
+        //                       32 x 2,048 sites   16 x 16,384   8 x 1,048,576
+        //   8 / 6 / 5 A set           41 / 14         42 / 18     1,107 / 183     (71 words, 2,103 members, 4 blocks)
+        //   pairs to 12 A             13 / 34         13 / 37       304 / 215     (229, 459, 3)
+        //   pairs 13 A, triplets 6    31 / 35         31 / 45       747 / 467     (301, 1,233, 2)
+        //   13 / 6 / 5 A set          56 / 41         56 / 56     1,403 / 630     (301, 2,565, 2)
+        //   pairs to 14.5 A           22 / 59         22 / 87       580 / 751     (443, 887, 1)
+        //   14.5 / 6 / 5 A set        64 / 55         64 / 104    1,585 / 1,291   (443, 2,849, 1)
+        //   16 / 6 / 5 A set          72 / 71         73 / 124    1,759 / 1,706   (578, 3,119, 1)
+        const int64_t per10 = fit == 1 ? (have < 4 * nsm ? 100 : 60) : fit == 2 && slices > 1 ? 21 : 10;
+        if (!h->bgrp || (h->erows && 10 * h->e_members < per10 * slices * h->e_words)) {
+            const int64_t rb = std::min<int64_t>((items + 255) / 256, 8192), rows_have = rb * h->nB * R;
+            const int rs = (int)std::max<int64_t>(1, std::min<int64_t>(32, (4ll * nsm + rows_have - 1) / rows_have));
+            ce_energy_rows_kernel<<<dim3((unsigned)(rb * rs), h->nB, R), 256, sizeof(unsigned long long) * h->n_cols, s>>>(
+                (const uint32_t *)planes.p, P, (int32_t)d0, (int32_t)d1, (int32_t)d2, W2, h->erows, h->emem, h->erow_off, h->erow_n,
+                h->n_cols, rs, (unsigned long long *)cv);
+        } else {
         auto kern = h->bw_oth == 3 ? (kw ? ce_energy_bits_kernel<3, 2> : ce_energy_bits_kernel<3, 1>)
                                    : (kw ? ce_energy_bits_kernel<7, 2> : ce_energy_bits_kernel<7, 1>);
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
