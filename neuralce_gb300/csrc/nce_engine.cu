@@ -76,6 +76,9 @@ struct NceDev {
     int32_t h0bits, h0_oth, h0_words, h0_wide; const uint4 *h0w; const int32_t *h0w_off; const uint32_t *h0row;
     const int32_t *h0grp;                     // (nB, C0 + 1) first group of each channel
     const float *h0lut; const int32_t *h0lut_off;   // (nB, C0 + 1)
+    // the same for the kernel that fetches every member: per basis, the rows' members as (basis, uo0, uo1, uo2) or basis -1,
+    // the weight of each channel, and slices of the rows (first row, first channel; the last (J, C0))
+    int32_t h0rows, h0_slices; const int4 *h0mem; const double *col_w; const int2 *h0_slice;  // (nB, h0_slices + 1)
     // tcgen05 layer contractions (mma 2: bf16, mma 4: split bf16): per layer the weights as the B operand in bf16
     // core-matrix layout ([D][Kp], Kp = Kin rounded up to 16; hi, then lo when split)
     int32_t tc, tc_split; const uint8_t *Wt[kMaxLayers];
@@ -1690,6 +1693,85 @@ __global__ void __launch_bounds__(32) nce_h0_bits_kernel(const __grid_constant__
     }
 }
 
+// grid (blocks, nB x S, R): threads over the (k0, k1, 32-site word) items of basis blockIdx.y / S, replica
+// blockIdx.z; slice blockIdx.y % S takes the rows and channels from its start to the next slice's (slices cut
+// the rows of a basis at channel boundaries, so small cells still fill the GPU).  Every member of every row is fetched
+// again, which is what bounds it; it keeps 2,048 threads an SM whatever the neighbourhood, so it is taken where few rows
+// share a word (nce_nce_full_cache).
+__global__ void __launch_bounds__(128) nce_h0_rows_kernel(const __grid_constant__ NceDev m, const uint32_t *__restrict__ planes, int32_t W2, float *h0) {
+    const int S = m.h0_slices, b = blockIdx.y / S, sl = blockIdx.y % S, r = blockIdx.z;
+    const int2 lo = m.h0_slice[b * (S + 1) + sl], hi = m.h0_slice[b * (S + 1) + sl + 1];   // (first row, first channel)
+    const int d0 = m.d0, d1 = m.d1, d2 = m.d2;
+    const int Wn = (d2 + 31) >> 5;
+    const int64_t items = (int64_t)d0 * d1 * Wn;
+    const int64_t it = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (it >= items) return;
+    const int w = (int)(it % Wn);
+    const int64_t kk = it / Wn;
+    const int k1 = (int)(kk % d1), k0 = (int)(kk / d1);
+    const int nv = min(32, d2 - 32 * w);
+    const uint32_t mask = nv >= 32 ? 0xffffffffu : ((1u << nv) - 1u);
+    const uint32_t *pr = planes + (int64_t)r * m.nB * d0 * d1 * W2;
+    const int C0 = m.C0;
+    // site j of the word: canonical index ((k0 d1 + k1) d2 + 32 w + j) nB + b
+    float *out0 = h0 + (((int64_t)r * m.N) + ((int64_t)(k0 * d1 + k1) * d2 + 32 * w) * m.nB + b) * C0;
+    const int64_t sstride = (int64_t)m.nB * C0;
+    if (m.Mb[b] < 2) {                                       // inactive sites: zeros
+        for (int j = 0; j < nv; ++j) for (int c = sl ? lo.y : 0; c < hi.y; ++c) out0[j * sstride + c] = 0.f;
+        return;
+    }
+    if (sl == 0) {
+        const float ch0 = (float)((1.0 - (double)m.mu[0]) / (double)m.sd[0]);
+        for (int j = 0; j < nv; ++j) out0[j * sstride] = ch0;
+    }
+    constexpr int NQ = 13;                                    // vertical counter planes: up to 8191 rows per channel
+    uint32_t cnt[NQ];
+    auto flush = [&](int ch, int nrows) {
+        const double wc = m.col_w[ch], base = (double)m.mu[ch] / (double)m.sd[ch];
+        for (int j = 0; j < nv; ++j) {
+            int odd = 0;
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) odd |= (int)((cnt[q] >> j) & 1u) << q;
+            out0[j * sstride + ch] = (float)((double)(nrows - 2 * odd) * wc - base);
+        }
+    };
+    int ch_cur = lo.y, nrows = 0;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) cnt[q] = 0u;
+    const int4 *mem = m.h0mem + (size_t)b * m.J * m.mo;
+    for (int jr = lo.x; jr < hi.x; ++jr) {
+        const int e = b * m.J + jr;
+        if (m.Rv_wfix[e] == 0) continue;
+        const int ch = m.Rv_col[e] + 1;
+        if (ch != ch_cur) {
+            flush(ch_cur, nrows);
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) cnt[q] = 0u;
+            for (int c = ch_cur + 1; c < ch; ++c) flush(c, 0);
+            ch_cur = ch; nrows = 0;
+        }
+        uint32_t par = 0;
+        for (int mm = 0; mm < m.mo; ++mm) {
+            const int4 d = mem[jr * m.mo + mm];                // (member basis or -1, uo0, uo1, uo2)
+            if (d.x < 0) continue;
+            int a0 = k0 + d.y; a0 -= a0 >= d0 ? d0 : 0;
+            int a1 = k1 + d.z; a1 -= a1 >= d1 ? d1 : 0;
+            const int pos = 32 * w + d.w;
+            const uint32_t *row = pr + (((int64_t)d.x * d0 + a0) * d1 + a1) * W2 + (pos >> 5);
+            par ^= __funnelshift_r(__ldg(row), __ldg(row + 1), (unsigned)(pos & 31));
+        }
+        // add the odd-parity bits into the vertical counter (ripple carry)
+        uint32_t carry = par & mask;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) { const uint32_t t = cnt[q] & carry; cnt[q] ^= carry; carry = t; }
+        ++nrows;
+    }
+    if (ch_cur < hi.y) flush(ch_cur, nrows);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) cnt[q] = 0u;
+    for (int c = ch_cur + 1; c < hi.y; ++c) flush(c, 0);
+}
+
 // Layer 0 of every site for general point functions: every reverse row of each site pulled in float64 (fixed
 // order, deterministic), standardised, float32
 __global__ void nce_h0_kernel(NceDev m, const int8_t *sigma, int32_t R, float *h0) {
@@ -1793,6 +1875,7 @@ struct nce_nce_model {
     std::mutex mu;
     int32_t *err = nullptr;
     std::vector<int32_t> h0grp, h0lut_off;      // host copies of dev.h0grp and dev.h0lut_off (slices of a launch)
+    int64_t h0_nwords = 0, h0_members = 0;      // distinct member offsets and members of all rows, over the bases
     // scratch for R replicas
     int32_t *slot = nullptr, *list = nullptr; float *newbuf = nullptr, *e_new = nullptr; int64_t stride = 0; int32_t R_alloc = 0;
     nce::NcePending *pend = nullptr;            // (R_alloc) swaps kept by nce_nce_local_delta
@@ -2147,6 +2230,26 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
             int oth = 0, most = 0, widest = 0;
             std::vector<std::vector<std::vector<std::vector<Mem>>>> by((size_t)d->nB, std::vector<std::vector<std::vector<Mem>>>((size_t)d->C0));
             std::vector<double> cwd((size_t)d->C0, 0.0);
+            // member by member: any rows on point function 0, sorted by channel
+            bool hr = hb;
+            std::vector<int4> hm(nr, make_int4(-1, 0, 0, 0));
+            for (int b = 0; b < d->nB; ++b) {
+                int last = 0, run = 0;
+                for (int j = 0; j < d->J && hr; ++j) {
+                    const size_t e = (size_t)b * d->J + j;
+                    if (wf[e] == 0) continue;
+                    const int ch = d->Rv_col[e] + 1;
+                    run = ch == last ? run + 1 : 1;
+                    hr = ch >= last && run <= 8191;
+                    last = ch;
+                    for (int k = 0; k < d->mo; ++k) {
+                        const size_t i = e * d->mo + k;
+                        if (!d->Rv_m[i]) continue;
+                        if (d->Rv_p[i] != 0) hr = false;
+                        hm[i] = make_int4(d->Rv_b[i], d->Rv_uo[3 * i], d->Rv_uo[3 * i + 1], d->Rv_uo[3 * i + 2]);
+                    }
+                }
+            }
             for (int b = 0; b < d->nB && hb; ++b)
                 for (int j = 0; j < d->J && hb; ++j) {
                     const size_t e = (size_t)b * d->J + j;
@@ -2201,7 +2304,46 @@ int nce_nce_create(const nce_nce_desc *d, nce_nce_handle *out) {
                 grp.push_back((int32_t)(rows.size() / (7 * (OT + 1))));
                 lut_off.push_back((int32_t)lut.size());
             }
+            h->h0_nwords = (int64_t)words.size();
+            for (const auto &x : by) for (const auto &c : x) for (const auto &r : c) h->h0_members += (int64_t)r.size() + 1;
             hb = hb && widest <= 700;
+            if (hr) {
+                for (int b = 0; b < d->nB; ++b)
+                    for (int j = 0; j < d->J; ++j)
+                        if (wf[(size_t)b * d->J + j] != 0) cwd[d->Rv_col[(size_t)b * d->J + j] + 1] = d->Rv_w[(size_t)b * d->J + j];
+                chk(dup(h, hm.data(), hm.size(), m.h0mem)); chk(dup(h, cwd.data(), cwd.size(), m.col_w));
+                // slices of each basis's rows, cut where the channel changes, about equal in rows
+                const int S = 8;
+                std::vector<int2> sl((size_t)d->nB * (S + 1));
+                for (int b = 0; b < d->nB; ++b) {
+                    std::vector<int> start_row, start_ch;            // candidate cuts: first row of each channel run
+                    int nrows = 0, last = -1;
+                    for (int j = 0; j < d->J; ++j) {
+                        const size_t e = (size_t)b * d->J + j;
+                        if (wf[e] == 0) continue;
+                        const int ch = d->Rv_col[e] + 1;
+                        if (ch != last) { start_row.push_back(j); start_ch.push_back(ch); last = ch; }
+                        ++nrows;
+                    }
+                    int2 *o = &sl[(size_t)b * (S + 1)];
+                    o[0] = make_int2(0, 1);
+                    int k = 1, seen = 0, ci = 0;
+                    for (int j = 0; j < d->J && k < S; ++j) {
+                        const size_t e = (size_t)b * d->J + j;
+                        if (wf[e] == 0) continue;
+                        while (ci < (int)start_row.size() && start_row[ci] < j) ++ci;
+                        if (ci < (int)start_row.size() && start_row[ci] == j && j > 0 && seen >= (int64_t)k * nrows / S &&
+                            start_ch[ci] > o[k - 1].y)
+                            o[k++] = make_int2(j, start_ch[ci]);
+                        ++seen;
+                    }
+                    for (; k <= S; ++k) o[k] = make_int2(d->J, d->C0);      // empty trailing slices
+                    o[S] = make_int2(d->J, d->C0);
+                }
+                chk(dup(h, sl.data(), sl.size(), m.h0_slice));
+                m.h0_slices = S;
+                m.h0rows = 1;
+            }
             if (hb) {
                 chk(dup(h, words.data(), words.size(), m.h0w)); chk(dup(h, word_off.data(), word_off.size(), m.h0w_off));
                 chk(dup(h, rows.data(), rows.size(), m.h0row)); chk(dup(h, grp.data(), grp.size(), m.h0grp));
@@ -2317,17 +2459,31 @@ int nce_nce_full_cache(nce_nce_handle h, const nce_nce_state *st, void *stream) 
         sm = sizeof(uint32_t) * 32 * (size_t)(m.h0_words + 1) + sizeof(float) * lut_max + (size_t)32 * nch * 36 * (m.h0_wide ? 2 : 1);
         if (S >= 16 || (int64_t)m.nB * S * 2 > 65535 || (sm <= 100 * 1024 && blocks * m.nB * st->R * S >= 8ll * nsm)) break;
     }
-    if (m.h0bits && st->R <= 65535 && sm <= 200 * 1024) {
+    // Words pay where each serves many rows, or while enough blocks fit an SM to hide the fetches' latency.  Kernel us, every
+    // member / words:                 32 x 2,048 sites   16 x 16,384   8 x 131,072
+    //   8 / 6 / 5 A set                   407 / 63          474 / 143    1,146 / 520     (141 words, 7,501 members)
+    //   pairs to 10 A                      51 / 45           79 / 75       157 / 143     (249, 497)
+    //   pairs to 11 A                      68 / 81           94 / 119      210 / 275     (369, 737)
+    //   11 / 6 / 5 A set                  398 / 160         452 / 283    1,378 / 1,111   (369, 7,957)
+    //   pairs to 12 A, triplets to 6 A    179 / 168         228 / 229      648 / 759     (459, 2,807)
+    //   pairs to 13 A                      83 / 199         122 / 293      325 / 613     (603, 1,205)
+    const bool words = m.h0bits && sm <= 200 * 1024 && (!m.h0rows || m.h0_words <= 300 || h->h0_members >= 8 * h->h0_nwords);
+    if ((words || m.h0rows) && st->R <= 65535) {
         const int32_t W2 = (2 * m.d2 + 31) / 32 + 1;
         StreamScratch planes;
         NCE_CUDA(planes.alloc(sizeof(uint32_t) * (size_t)st->R * m.nB * m.d0 * m.d1 * W2, s));
         const int64_t prow = (int64_t)st->R * m.nB * m.d0 * m.d1;
         nce_plane_kernel<<<(int)std::min<int64_t>((prow + 7) / 8, 1 << 20), 256, 0, s>>>(m, st->sigma, st->R, W2, (uint32_t *)planes.p);
         NCE_CUDA(cudaGetLastError());
+        if (!words) {
+            nce_h0_rows_kernel<<<dim3((unsigned)((items + 127) / 128), m.nB * m.h0_slices, st->R), 128, 0, s>>>(
+                m, (const uint32_t *)planes.p, W2, st->h0);
+        } else {
         auto kern = m.h0_wide ? (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 13, uint16_t> : nce_h0_bits_kernel<7, 13, uint16_t>)
                               : (m.h0_oth == 3 ? nce_h0_bits_kernel<3, 8, uint8_t> : nce_h0_bits_kernel<7, 8, uint8_t>);
         NCE_CUDA(::nce::raise_smem_limit((const void *)kern, sm));
         kern<<<dim3((unsigned)blocks, m.nB * S, st->R), 32, sm, s>>>(m, (const uint32_t *)planes.p, W2, S, lut_max, st->h0);
+        }
     } else {
         nce_h0_kernel<<<(int)std::min<int64_t>((tot + 127) / 128, 65535), 128, 0, s>>>(m, st->sigma, st->R, st->h0);
     }
