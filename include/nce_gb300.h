@@ -172,7 +172,8 @@ typedef struct {
     const double *ex_u;        /* (ceil((R-1)/2)) device uniforms, or NULL -> Philox */
     int32_t precision;         /* 64 or 32 */
     int32_t warps;             /* warps per replica (0 = default); the windowed sign-parity kernel (one basis site per
-                                  cell) has a launch shape of its own and ignores warps and cluster */
+                                  cell) has a launch shape of its own and ignores warps and cluster
+                                  (nce_ce_chunk_kernel) */
     int32_t path;              /* 0 auto (local field when the state has a field, else sign parity when the point
                                   functions are in {-1,+1}, else general), 1 general point-function products, 2 sign
                                   parity, 3 local field (precision 64, state.field set) */
@@ -191,6 +192,14 @@ int nce_ce_run_chunk(nce_ce_handle h, const nce_pt_state *st, const nce_pt_chunk
  * Every chunk in the batch must use the same precision and warps. */
 int nce_ce_run_batch(int32_t n_jobs, const nce_ce_handle *h, const nce_pt_state *st, const nce_pt_chunk *ck,
                      void *stream);
+
+/* The kernel that a chunk of these jobs takes together, as nce_ce_run_batch (one job: nce_ce_run_chunk) chooses it:
+ * NCE_CE_WINDOWED has a launch shape of its own (one CTA a replica, `threads` threads) and ignores the chunk's warps and
+ * cluster; the others take them (cluster: NCE_CE_SIGN_PARITY alone).  states may be NULL (no field, no tracked sums; threads
+ * is then 0).  threads may be NULL and is 0 for the other kernels. */
+enum { NCE_CE_GENERAL = 1, NCE_CE_SIGN_PARITY = 2, NCE_CE_LOCAL_FIELD = 3, NCE_CE_WINDOWED = 4 };
+int nce_ce_chunk_kernel(int32_t n_jobs, const nce_ce_handle *h, const nce_pt_state *states, int32_t precision, int32_t path,
+                        int32_t *kernel, int32_t *threads);
 
 /* e2e form: the same chunk with HOST buffers.  sigma_host (R,N), E_host (R) and the permutations are read
  * and written back; prop_* are host arrays (or NULL for Philox); E_samples_host (n_steps/si, R) receives

@@ -100,6 +100,7 @@ SIGNATURES = {
     "nce_ce_cluster_counts": (i32, [vp, vp, i32, vp, vp]),
     "nce_ce_energy_from_counts": (i32, [vp, vp, i32, vp, vp]),
     "nce_ce_run_batch": (i32, [i32, P(vp), P(NcePtState), P(NcePtChunk), vp]),
+    "nce_ce_chunk_kernel": (i32, [i32, P(vp), P(NcePtState), i32, i32, P(i32), P(i32)]),
     "nce_ce_run_chunk_host": (i32, [vp, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, P(NcePtChunk), vp]),
     "nce_ce_errors": (i32, [vp, P(i32)]),
     "nce_ce_field_init": (i32, [vp, vp, i32, vp, vp]),

@@ -1,12 +1,13 @@
 """Launch-shape autotuner of the CE chunk kernels: warps per CTA, CTAs per replica (thread-block cluster) and,
 optionally, the kernel (sign parity or local field).
 
-Per-step latency, not throughput, bounds a Markov chain, and the best shape depends on the number of rows per
-site, the replica count relative to the 152 SMs and the precision: with few replicas, spreading each replica
-over a cluster of 2-8 CTAs puts idle SMs to work on the row phase at the price of one cluster barrier per
-evaluated swap.  The tuner times a short chunk of the real kernel for each candidate on a scratch copy of the
-state (the job's own state is untouched) and keeps the fastest; results are cached per (tables, R, precision,
-path); the key names the model by its serial number, which no later model reuses."""
+The step-by-step kernels are bound by per-step latency, and their best shape depends on the number of rows per site, the
+replica count relative to the 152 SMs and the precision: with few replicas, spreading each replica over a cluster of 2-8
+CTAs puts idle SMs to work on the row phase at the price of one cluster barrier per evaluated swap.  The tuner times a
+short chunk of the real kernel for each candidate on a scratch copy of the state (the job's own state is untouched) and
+keeps the fastest; results are cached per (tables, R, precision, path); the key names the model by its serial number,
+which no later model reuses.  The windowed kernel has a launch shape of its own and ignores both numbers: it is timed
+once, under the first candidate."""
 from __future__ import annotations
 
 _cache = {}
@@ -19,7 +20,7 @@ def best_launch(gce, st, precision=64, path=0, warps=(2, 4, 8, 16, 32), clusters
     {(warps, cluster, path): ms})."""
     import torch
     from . import _lib
-    from .pt import PTState, run_chunk
+    from .pt import PTState, chunk_kernel, run_chunk
     key = (gce.serial, st.R, precision, path, tuple(warps), tuple(clusters), tuple(paths or ()))
     if key in _cache:
         return _cache[key]
@@ -40,6 +41,11 @@ def best_launch(gce, st, precision=64, path=0, warps=(2, 4, 8, 16, 32), clusters
         clusters = (1,)                                   # one CTA per replica: the decider warp is the chain
         warps = tuple(w for w in warps if w <= 16) or (16,)   # the kernel's CTAs hold at most 16 warps
     timings = {}
+    try:
+        if chunk_kernel([gce], [scratch], precision, path)[0] == "windowed":
+            warps, clusters = warps[:1], (1,) if 1 in clusters else clusters[:1]
+    except _lib.NceError:
+        pass                                              # (a path that cannot run fails below, candidate by candidate)
     for cl in clusters:
         for w in warps:
             try:

@@ -12,7 +12,7 @@ import ctypes as C
 import numpy as np
 
 from . import _lib
-from .pt import PTState, make_chunk
+from .pt import PTState, chunk_kernel, make_chunk
 
 MAX_JOBS = 64
 SPLIT_SITES = 48 * 1024       # a job whose occupancy fits the batch kernel's per-job shared memory can be split over CTAs
@@ -48,10 +48,21 @@ class CEBatch:
             idx = [(g, c) for g, c in ((small, self.cluster), (large, 1)) if g]
         return [(g[a:a + MAX_JOBS], c) for g, c in idx for a in range(0, len(g), MAX_JOBS)]
 
+    def _launches(self):
+        """launch_groups, but for the windowed kernel, which ignores a split: its jobs need no launch of their own"""
+        groups = self.launch_groups()
+        if self.cluster > 1 and len(groups) > 1 and len({j["gce"].max_size for j in self.jobs}) == 1:
+            idx = list(range(len(self.jobs)))
+            parts = [idx[a:a + MAX_JOBS] for a in range(0, len(idx), MAX_JOBS)]
+            if all(chunk_kernel([self.jobs[k]["gce"] for k in p], [self.states[k] for k in p], self.precision, self.path)[0]
+                   == "windowed" for p in parts):
+                return [(p, 1) for p in parts]
+        return groups
+
     def run_chunk(self, n_steps, do_exchange=True, stream=None, step_dev=None):
         """one chunk of every job (launch_groups).  step_dev: (n_jobs,) int64 device step counters that the launch
         reads and advances (used inside captured graphs) instead of the host step."""
-        for js, cl in self.launch_groups():
+        for js, cl in self._launches():
             n = len(js)
             hs = (C.c_void_p * n)(*[self.jobs[k]["gce"].handle.value for k in js])
             ss = (_lib.NcePtState * n)(*[self.states[k].struct() for k in js])
@@ -116,9 +127,12 @@ class CEBatch:
 
 def tune_launch(jobs, precision=32, warps=(4, 8, 16, 32), clusters=(1, 2, 4), steps=200):
     """Autotune a batch's launch shape, warps per CTA and the split (CTAs per replica of the jobs that can be split):
-    time a short chunk of the real batch for each candidate on scratch states.  Returns ((warps, cluster), {...: ms})."""
+    time a short chunk of the real batch for each candidate on scratch states.  Returns ((warps, cluster), {...: ms}).
+    A batch that runs on the windowed kernel throughout, which ignores both, is timed once, under the first candidate."""
     import torch
     times = {}
+    if all(chunk_kernel([j["gce"] for j in jobs[a:a + MAX_JOBS]], None, precision)[0] == "windowed" for a in range(0, len(jobs), MAX_JOBS)):
+        warps, clusters = warps[:1], (1,) if 1 in clusters else clusters[:1]
     for cl in clusters:
         for w in warps:
             b = CEBatch(jobs, precision, w, track=False, cluster=cl)

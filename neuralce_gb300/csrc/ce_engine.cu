@@ -1823,6 +1823,56 @@ static int check_chunk(const nce_pt_state *st, const nce_pt_chunk *ck) {
     return NCE_OK;
 }
 
+// The kernel that a chunk of these jobs runs together.  sts may be null (no field, no tracked sums).
+static int choose_kernel(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *sts, int precision, int path, int *kernel) {
+    bool all_bin = true;
+    for (int j = 0; j < n_jobs; ++j) all_bin = all_bin && hs[j]->binary;
+    NCE_CHECK(path >= 0 && path <= 3, "chunk: path must be 0 (auto), 1 (general), 2 (sign parity) or 3 (local field)");
+    NCE_CHECK(path < 2 || all_bin, "chunk: the sign-parity and local-field paths need point functions in {-1, +1}");
+    // local field: every job has its tables and a field buffer, float64 (fixed-point) arithmetic
+    bool all_lf = precision == 64;
+    for (int j = 0; j < n_jobs; ++j) all_lf = all_lf && hs[j]->lf_ok && sts && sts[j].field != nullptr;
+    if (path == 3) {
+        for (int j = 0; j < n_jobs; ++j) {
+            NCE_CHECK(hs[j]->lf_ok, "chunk: the local-field path is not available for this cell (aliasing neighbourhood "
+                                    "or tables too large)");
+            NCE_CHECK(sts && sts[j].field, "chunk: the local-field path needs the state's field buffer (nce_ce_field_init)");
+        }
+        NCE_CHECK(precision == 64, "chunk: the local-field path computes in fixed point (precision 64)");
+    }
+    const bool use_lf = path == 3 || (path == 0 && all_lf);
+    // the float64 sign-parity kernel sums in fixed point: a table whose column eci allow no exact fixed point (never
+    // for eci of physical size) runs the general kernel
+    bool all_fix = true;
+    for (int j = 0; j < n_jobs; ++j) all_fix = all_fix && hs[j]->fix_shift > 0;
+    NCE_CHECK(!(path == 2 && precision == 64 && !all_fix),
+              "chunk: the float64 sign-parity path needs fixed-point column eci (2 J max|eci| below 2^41)");
+    const bool use_bin = !use_lf && ((path == 2) || (path == 0 && all_bin && (precision == 32 || all_fix)));
+    for (int j = 0; j < n_jobs; ++j)
+        NCE_CHECK(!sts || !sts[j].cv || use_bin || use_lf, "chunk: tracked cluster-vector sums need the sign-parity or local-field path");
+    // windowed kernel wherever the sign-parity path runs and every job has its tables (build_window_tables): it was faster
+    // at every size, ladder and cluster set measured, against the step-by-step kernel at its best launch shape (2,048 sites
+    // x 32 replicas, 1,000 steps: 1,232 -> 211 us; 131,072 x 256, 300 steps: 1,460 -> 112 us; 256 x 16, 10 steps: 77 -> 23 us;
+    // 24 float32 jobs of 256 to 32,000 sites, 500 steps: 4,268 -> 672 us; pairs to 4 A, 256 x 4, 1,000 steps: 805 -> 250 us;
+    // 14.5 / 6 / 5 A set, 2,048 x 600, 200 steps: 1,488 -> 385 us).  warps and cluster only shape the step-by-step
+    // kernels, which keep the other tables (several basis sites, larger orders, one-cell images).
+    bool use_win = use_bin;
+    for (int j = 0; j < n_jobs; ++j) use_win = use_win && hs[j]->win != nullptr;
+    *kernel = use_win ? NCE_CE_WINDOWED : use_lf ? NCE_CE_LOCAL_FIELD : use_bin ? NCE_CE_SIGN_PARITY : NCE_CE_GENERAL;
+    return NCE_OK;
+}
+
+// Threads a CTA of the windowed kernel, one CTA a replica.
+static int win_threads_for(int total) {
+    // many replicas: four CTAs of 256 threads an SM instead of two of 512 keep more windows in flight between
+    // the barriers (24 jobs, about 900 replicas: 720 -> 674 us); with fewer a window takes longer than it gains (131,072
+    // sites x 256, an earlier state of the kernel: 119 us with 512 threads, 136 with 256)
+    int dev = 0, n_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    return total >= 3 * n_sm ? 256 : 512;
+}
+
 static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *sts, const nce_pt_chunk *cks, cudaStream_t s) {
     NCE_CHECK(n_jobs >= 1 && n_jobs <= kMaxJobs, "batch: n_jobs must be 1..%d", kMaxJobs);
     const int precision = cks[0].precision;
@@ -1840,55 +1890,19 @@ static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *st
     for (int j = 0; j < n_jobs; ++j)
         NCE_CHECK(hs[j]->mo == mo, "batch: all jobs must have the same maximum cluster order");
     const int path = cks[0].path;
-    bool all_bin = true;
-    for (int j = 0; j < n_jobs; ++j) {
-        NCE_CHECK(cks[j].path == path, "batch: all chunks must use the same path");
-        all_bin = all_bin && hs[j]->binary;
-    }
-    NCE_CHECK(path >= 0 && path <= 3, "chunk: path must be 0 (auto), 1 (general), 2 (sign parity) or 3 (local field)");
-    NCE_CHECK(path < 2 || all_bin, "chunk: the sign-parity and local-field paths need point functions in {-1, +1}");
-    // local field: every job has its tables and a field buffer, float64 (fixed-point) arithmetic
-    bool all_lf = precision == 64;
-    for (int j = 0; j < n_jobs; ++j) all_lf = all_lf && hs[j]->lf_ok && sts[j].field != nullptr;
-    if (path == 3) {
-        for (int j = 0; j < n_jobs; ++j) {
-            NCE_CHECK(hs[j]->lf_ok, "chunk: the local-field path is not available for this cell (aliasing neighbourhood "
-                                    "or tables too large)");
-            NCE_CHECK(sts[j].field, "chunk: the local-field path needs the state's field buffer (nce_ce_field_init)");
-        }
-        NCE_CHECK(precision == 64, "chunk: the local-field path computes in fixed point (precision 64)");
-    }
-    const bool use_lf = path == 3 || (path == 0 && all_lf);
-    // the float64 sign-parity kernel sums in fixed point: a table whose column eci allow no exact fixed point (never
-    // for eci of physical size) runs the general kernel
-    bool all_fix = true;
-    for (int j = 0; j < n_jobs; ++j) all_fix = all_fix && hs[j]->fix_shift > 0;
-    NCE_CHECK(!(path == 2 && precision == 64 && !all_fix),
-              "chunk: the float64 sign-parity path needs fixed-point column eci (2 J max|eci| below 2^41)");
-    const bool use_bin = !use_lf && ((path == 2) || (path == 0 && all_bin && (precision == 32 || all_fix)));
-    for (int j = 0; j < n_jobs; ++j)
-        NCE_CHECK(!sts[j].cv || use_bin || use_lf, "chunk: tracked cluster-vector sums need the sign-parity or local-field path");
+    for (int j = 0; j < n_jobs; ++j) NCE_CHECK(cks[j].path == path, "batch: all chunks must use the same path");
+    int kernel = 0;
+    int crc = choose_kernel(n_jobs, hs, sts, precision, path, &kernel);
+    if (crc) return crc;
+    const bool use_lf = kernel == NCE_CE_LOCAL_FIELD, use_win = kernel == NCE_CE_WINDOWED, use_bin = kernel == NCE_CE_SIGN_PARITY || use_win;
     CEBatch bt; std::memset(&bt, 0, sizeof(bt));
     bt.n_jobs = n_jobs;
     size_t smem = 0; bool all_fit = true;
     int sig_smem = 0;
     int64_t lf_budget = 0;
-    // windowed kernel wherever the sign-parity path runs and every job has its tables (build_window_tables): it was faster
-    // at every size and ladder measured, against the step-by-step kernel at its best launch shape (2,048 sites x 32
-    // replicas, 1,000 steps: 1,202 -> 211 us; 131,072 x 256, 300 steps: 1,196 -> 112 us; 256 x 16, 10 steps: 63 -> 23 us;
-    // 24 float32 jobs of 256 to 32,000 sites, 500 steps: 4,154 -> 722 us).  warps and cluster only shape the
-    // step-by-step kernels, which keep the other tables (several basis sites, larger orders, one-cell images).
-    bool use_win = use_bin;
-    for (int j = 0; j < n_jobs; ++j) use_win = use_win && hs[j]->win != nullptr;
-    int win_threads = 512;
+    int win_threads = 0;
     if (use_win) {
-        // many replicas: four CTAs of 256 threads an SM instead of two of 512 keep more windows in flight between
-        // the barriers (24 jobs, about 900 replicas: 720 -> 674 us); with fewer a window takes longer than it gains (131,072
-        // sites x 256, an earlier state of the kernel: 119 us with 512 threads, 136 with 256)
-        int dev = 0, n_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-        if (total >= 3 * n_sm) win_threads = 256;
+        win_threads = win_threads_for(total);
         for (int j = 0; j < n_jobs; ++j) {
             const WinTab &w = hs[j]->win_host;
             smem = std::max(smem, WinLayout::make(w.n_ent, w.n_blk, hs[j]->n_cols).total);
@@ -2763,6 +2777,23 @@ int nce_ce_run_chunk(nce_ce_handle h, const nce_pt_state *st, const nce_pt_chunk
 int nce_ce_run_batch(int32_t n_jobs, const nce_ce_handle *hs, const nce_pt_state *st, const nce_pt_chunk *ck, void *stream) {
     NCE_CHECK(hs && st && ck, "nce_ce_run_batch: null argument");
     return run_batch(n_jobs, hs, st, ck, (cudaStream_t)stream);
+}
+
+int nce_ce_chunk_kernel(int32_t n_jobs, const nce_ce_handle *hs, const nce_pt_state *sts, int32_t precision, int32_t path,
+                        int32_t *kernel, int32_t *threads) {
+    NCE_CHECK(n_jobs >= 1 && n_jobs <= kMaxJobs && hs && kernel, "nce_ce_chunk_kernel: bad argument");
+    for (int j = 0; j < n_jobs; ++j) NCE_CHECK(hs[j], "nce_ce_chunk_kernel: null handle");
+    NCE_CHECK(precision == 64 || precision == 32, "nce_ce_chunk_kernel: precision must be 64 or 32");
+    int k = 0;
+    int rc = choose_kernel(n_jobs, hs, sts, precision, path, &k);
+    if (rc) return rc;
+    *kernel = k;
+    if (threads) {
+        int total = 0;
+        for (int j = 0; j < n_jobs && sts; ++j) total += sts[j].R;
+        *threads = k == NCE_CE_WINDOWED && sts ? win_threads_for(total) : 0;
+    }
+    return NCE_OK;
 }
 
 int nce_pt_minimum(const nce_pt_state *st, double *out_min, int32_t *out_arg, void *stream) {

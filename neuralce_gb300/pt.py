@@ -176,6 +176,21 @@ def make_chunk(n_steps, step0, seed, precision=64, warps=0, proposals=None, samp
     return c
 
 
+CHUNK_KERNELS = {1: "general", 2: "sign parity", 3: "local field", 4: "windowed"}
+
+
+def chunk_kernel(gces, states=None, precision=64, path=0):
+    """(kernel, threads) that a chunk of these jobs takes together: "general", "sign parity", "local field" or "windowed"
+    (``nce_ce_chunk_kernel``).  The windowed kernel runs one CTA of ``threads`` threads a replica whatever the chunk's warps
+    and cluster; for the others threads is 0."""
+    n = len(gces)
+    hs = (C.c_void_p * n)(*[g.handle.value for g in gces])
+    ss = (_lib.NcePtState * n)(*[s.struct() for s in states]) if states is not None else None
+    k, t = C.c_int32(0), C.c_int32(0)
+    _lib.check(_lib.lib().nce_ce_chunk_kernel(n, hs, ss, int(precision), int(path), C.byref(k), C.byref(t)), "nce_ce_chunk_kernel")
+    return CHUNK_KERNELS[k.value], t.value
+
+
 def run_chunk(gce, st: PTState, n_steps, step0, seed, precision=64, warps=0, proposals=None, sample_interval=1,
               E_samples=None, do_exchange=False, ex_parity=0, ex_u=None, stream=None, path=0, cluster=1, near_eV=0.0):
     """One chunk of the persistent kernel (+ chunk-end exchange) for one job.  path: 0 auto (local field when the state
