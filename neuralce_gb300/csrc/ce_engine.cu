@@ -1864,13 +1864,15 @@ static int choose_kernel(int n_jobs, const nce_ce_handle *hs, const nce_pt_state
 
 // Threads a CTA of the windowed kernel, one CTA a replica.
 static int win_threads_for(int total) {
-    // many replicas: four CTAs of 256 threads an SM instead of two of 512 keep more windows in flight between
-    // the barriers (24 jobs, about 900 replicas: 720 -> 674 us); with fewer a window takes longer than it gains (131,072
-    // sites x 256, an earlier state of the kernel: 119 us with 512 threads, 136 with 256)
+    // more replicas than two CTAs of 512 threads an SM hold: four of 256 keep all of them in flight; up to that a window takes
+    // longer than it gains.  us of 300 steps with 512 / 256 threads (2,048 sites, 8 / 6 / 5 A set, float64): 160 replicas 128 /
+    // 142, 304 137 / 146, 320 179 / 162, 456 214 / 168, 608 233 / 209, 912 333 / 308, 1,824 620 / 515; float32 138 / 147 at
+    // 304, 191 / 163 at 320; 131,072 sites 113 / 124, 154 / 139; pairs to 6 A 108 / 107, 151 / 112; 14.5 / 6 / 5 A set (two
+    // CTAs of either size an SM) 321 / 361, 415 / 420, 456 / 441 at 456.
     int dev = 0, n_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
-    return total >= 3 * n_sm ? 256 : 512;
+    return total > 2 * n_sm ? 256 : 512;
 }
 
 static int run_batch(int n_jobs, const nce_ce_handle *hs, const nce_pt_state *sts, const nce_pt_chunk *cks, cudaStream_t s) {

@@ -53,8 +53,8 @@ def test_which_kernel(cuda):
         for path in (0, 2):
             assert chunk_kernel([fcc], [st], prec, path) == ("windowed", 512)
     assert chunk_kernel([fcc]) == ("windowed", 0)
-    many = _state(cuda, fcc, np.repeat(sig[:1], 3 * n_sm, 0))
-    assert chunk_kernel([fcc], [many]) == ("windowed", 256)
+    many = _state(cuda, fcc, np.repeat(sig[:1], 2 * n_sm, 0))
+    assert chunk_kernel([fcc], [many]) == ("windowed", 512)
     assert chunk_kernel([fcc, fcc], [many, st]) == ("windowed", 256)
     st.cv = None
     assert chunk_kernel([fcc], [st], 64, 1) == ("general", 0)
