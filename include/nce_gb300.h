@@ -278,7 +278,8 @@ typedef struct nce_nce_model *nce_nce_handle;
 typedef struct {
     int32_t R; int64_t N;
     int8_t *sigma;         /* (R, N) */
-    float *h0;             /* (R, N, C0) standardised layer 0 */
+    float *h0;             /* (R, N, C0) standardised layer 0; 8-byte aligned where C0 is even (any float alignment on the
+                              tcgen05 forms) */
     float *hmid;           /* (depth-1, R, N, D) hidden layers 1..depth-1, or NULL for depth < 2 */
     float *e;              /* (R, N) per-site energy */
     double *E;             /* (R) energy: sum(e)/norm + head_b */

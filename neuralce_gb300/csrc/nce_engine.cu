@@ -360,12 +360,6 @@ struct LayerW {            // weights of one layer as seen by the kernel (shared
     const float *W, *b, *G, *gb;
 };
 
-// Evaluate one layer for the sites list[pos0 .. pos0+cnt), or (direct0) the rows *direct0 + 0..cnt-1 of all replicas'
-// caches, row r N + s being site s of replica r.  Inputs come from level lvl
-// (cache patched with the step's values, or unpatched when slot == nullptr).  For every site and group of 4
-// consecutive output columns, `sink(pos, col0, v[4])` receives the activated outputs (pos < 0: padding lane); with head
-// weights ehw, the tiles sum each site's energy themselves (head terms, then the linear term of the layer-0 row
-// esink.row(pos, site, slot), as site_energy does) and hand it to esink.done(pos, site, energy).
 // sum over the D/4 lanes of one site (consecutive lanes of one warp)
 __device__ __forceinline__ float group_sum(float v, int ncg) {
     for (int o = ncg >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, ncg);
@@ -382,6 +376,12 @@ struct NoSink {
     __device__ void done(int64_t, int32_t, float) const {}
 };
 
+// Evaluate one layer for the sites list[pos0 .. pos0+cnt), or (direct0) the rows *direct0 + 0..cnt-1 of all replicas'
+// caches, row r N + s being site s of replica r.  Inputs come from level lvl
+// (cache patched with the step's values, or unpatched when slot == nullptr).  For every site and group of 4
+// consecutive output columns, `sink(pos, col0, v[4])` receives the activated outputs (pos < 0: padding lane); with head
+// weights ehw, the tiles sum each site's energy themselves (head terms, then the linear term of the layer-0 row
+// esink.row(pos, site, slot), as site_energy does) and hand it to esink.done(pos, site, energy).
 // (TC: the tcgen05 tiles, tc set.  The two forms are compiled apart: in one body the float32 form of the shipped model ran 10%
 // slower, 2,306 -> 2,580 us for 40 steps of 32 replicas)
 template <bool TC, typename Sink, typename ESink = NoSink>
@@ -405,9 +405,8 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
     int4 *tk = reinterpret_cast<int4 *>(tinv + TM);          // (basis, k0, k1, k2) of each
     int32_t *tslot = reinterpret_cast<int32_t *>(tk + TM);   // slot-map value of each (-1: not in the field)
     // tcgen05 path: the tile is the bf16 A operand [128][KS] (hi, then lo when split) in core-matrix layout, one K
-    // slice [klo, klo + KS) of the layer's Kp input columns at a time (KS = Kp unless the whole A operand does not
-    // fit shared memory: the split form at width 128 takes its self channels, then its shell means); every slice's
-    // MMAs accumulate into the same tensor-memory tile
+    // slice [klo, klo + KS) of at most kTcSlice of the layer's Kp input columns at a time; every slice's MMAs
+    // accumulate into the same tensor-memory tile
     const int Kp = kpad16(Kin);
     const int KS = (tc && Kp > m.tc_ks) ? m.tc_ks : Kp, nks = (Kp + KS - 1) / KS;   // (the last slice may be narrower)
     int klo = 0, khi = Kp;                                   // the slice being gathered (all of K off the tcgen05 path)
