@@ -9,8 +9,10 @@ the whole job is 40 such steps.  Proposals come from the device Philox stream.
   value     swap attempts/s with the state resident in HBM, CUDA events around each chunk on its stream,
             L2 flushed (256 MB write) between timed chunks outside the events
   e2e       the same chunks through nce_ce_run_chunk_host: pinned host buffers in and out every chunk
-  roofline  dominant kernel ce_win_chunk_kernel (windowed sign-parity form); algorithmic bytes per attempt = 14,996 B
-            of int8 member-occupancy reads (2 x 7,498 member slots of the rows of both sites)
+  roofline  dominant kernel ce_win_chunk_kernel (windowed sign-parity form), bound by the latency of its windows; bytes a chunk
+            cannot do without: the int8 neighbourhoods of both sites of every swap between different species, each
+            byte of the occupancies read and written once at most (the step-by-step kernels: 14,996 B of member reads
+            an attempt, 2 x 7,498 member slots of the rows of both sites)
   cpu_baseline  the oracle's C restatement on the host cores (bounded sample, all threads)
   side lines  nce (configuration 1, float32), nce_tcgen05_split / nce_tcgen05_bf16 (the same on tcgen05
             tensor cores), nce_shipped_model (the reference's shipped PtNi model on the same cell), batch
@@ -38,12 +40,31 @@ CONTRACTIONS = ["fp32 CUDA cores", "bf16 mma.sync tensor cores (fp32 accumulatio
                 "bf16 tcgen05 tensor cores (fp32 accumulation in tensor memory)", "split-bf16 mma.sync tensor cores",
                 "split-bf16 tcgen05 tensor cores"]
 H100_PUBLISHED = 1_231_993.0          # reference CE PT, 2,048 sites, R=32, H100 (results/bench_stage/gpu_icet_*H100*.json)
-B_GATHER = 14_996                     # bytes of member occupancy per attempt, config-0 cluster set
-# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from one ncu capture of the headline kernel,
-# keyed by (path, L, R, steps per chunk): profiles/ holds the capture (a 1000-step chunk; the tables and occupancy
-# are read once per launch, so the figure does not grow with the steps)
-TRAFFIC = {(2, 8, 32, 5000): 159_744}
-SMEM_PIPE = {(2, 8, 32, 5000): 0.040}       # the same capture's shared-memory wavefronts, fraction of the pipe's peak
+B_GATHER = 14_996                     # bytes of member occupancy per attempt of the step-by-step kernels, 8 / 6 / 5 A set
+CE_KERNELS = {"general": "ce_pt_chunk_kernel", "sign parity": "ce_bin_chunk_kernel", "local field": "ce_lf_chunk_kernel",
+              "windowed": "ce_win_chunk_kernel"}
+# DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) of the windowed kernel from an ncu capture of a
+# 1,000-step chunk of 2,048 sites x 32 replicas (profiles/window_energy_cache_kernels.txt; the tables and occupancies are read
+# once per launch, so the figure does not grow with the steps), keyed by (kernel, L, R)
+TRAFFIC = {("windowed", 8, 32): 158_720}
+SMEM_PIPE = {("windowed", 8, 32): 0.050}    # the same capture's shared-memory wavefronts, fraction of the pipe's peak
+
+
+def ce_chunk_bytes(gce, kernel, R, T, x_pt=0.5):
+    """Bytes that one chunk of T steps cannot do without (occupancy reads and writes; the tables stay on chip).  Windowed: the
+    neighbourhoods of both sites of every swap between different species, every byte of the state at most once each way.
+    Step by step: the members of the rows of both sites at every attempt."""
+    if kernel != "windowed":
+        return R * T * B_GATHER
+    swaps, state = 2.0 * x_pt * (1.0 - x_pt) * T * R, R * gce.n_atoms
+    return int(min(swaps * 2 * gce.info["n_nbr"], state) + min(swaps * 2, state))
+
+
+def ce_launch(kernel, threads, warps, cluster):
+    """the launch shape that ran: the windowed kernel has one of its own"""
+    if kernel == "windowed":
+        return {"kernel": CE_KERNELS[kernel], "warps_per_cta": threads // 32, "ctas_per_replica": 1}
+    return {"kernel": CE_KERNELS[kernel], "warps_per_cta": warps or 8, "ctas_per_replica": max(1, cluster)}
 
 
 def parse():
@@ -295,7 +316,7 @@ def bench_batch(steps=3, warmup=1, chunk=5000, reanchor=10000, n_jobs=64, alone_
     cluster-vector sums.  Compared with the plain float64 kernels running the first ``alone_jobs`` jobs alone."""
     import torch
     from neuralce_gb300.batch import CEBatch, tune_launch
-    from neuralce_gb300.pt import PTState, run_chunk
+    from neuralce_gb300.pt import PTState, chunk_kernel, run_chunk
     from neuralce_gb300.workloads import ce_batch_config
     from neuralce_gb300.autotune import best_warps
     t0 = time.time()
@@ -334,6 +355,10 @@ def bench_batch(steps=3, warmup=1, chunk=5000, reanchor=10000, n_jobs=64, alone_
             torch.cuda.synchronize()
             secs += a_.elapsed_time(c_) / 1e3; att += j["R"] * alone_steps
         alone[path] = att / secs
+    shape = []
+    for a in range(0, len(jobs), 64):
+        k_, t_ = chunk_kernel([j["gce"] for j in jobs[a:a + 64]], b.states[a:a + 64], 32)
+        shape.append(ce_launch(k_, t_, w, cl))
     return {"value": value, "unit": "swap attempts/s", "ms_per_step": 1e3 * tot / steps,
             "config": f"{n_jobs} CE jobs, one CUDA graph per {b._graph_steps} steps: L~U{{4..32}} "
                       f"({min(j['N'] for j in jobs)}-{max(j['N'] for j in jobs)} sites), x_Pt~U[0.1,0.9], R~U{{16,32,64}} "
@@ -342,8 +367,7 @@ def bench_batch(steps=3, warmup=1, chunk=5000, reanchor=10000, n_jobs=64, alone_
             "fp64_single_job_alone": alone[1], "ratio_vs_fp64_single_job": value / alone[1],
             "fp64_sign_parity_single_job_alone": alone[2], "ratio_vs_fp64_sign_parity_single_job": value / alone[2],
             "max_fp32_drift_before_reanchor_eV": drift, "max_reanchored_vs_full_recompute_eV": full_err,
-            "warps_per_replica": w, "ctas_per_replica_of_split_jobs": cl,
-            "autotune_ms": {f"{a}x{b_}": round(v, 3) for (a, b_), v in tune.items()}, "setup_s": setup}
+            "launches": shape, "autotune_ms": {f"{a}x{b_}": round(v, 3) for (a, b_), v in tune.items()}, "setup_s": setup}
 
 
 def bench_serve(seconds=10.0, rate=50.0, ce_scale=0.01, nce_scale=0.0002, nce_max_sites=32768, seed=4, alone_jobs=0,
@@ -357,7 +381,7 @@ def bench_serve(seconds=10.0, rate=50.0, ce_scale=0.01, nce_scale=0.0002, nce_ma
     limits that to the first jobs; 0 = all).  NeuralCE jobs run the precision form ``nce_mma`` (4: split bf16 operands on
     the tcgen05 tensor cores, float32 accumulation, within 1e-4 eV per swap; 2: plain bf16)."""
     import torch
-    from neuralce_gb300.pt import PTState, run_chunk
+    from neuralce_gb300.pt import PTState, chunk_kernel, run_chunk
     from neuralce_gb300.serve import Server
     from neuralce_gb300.workloads import ServeModels, ladder, random_occupancy, serve_stream
     t0 = time.time()
@@ -384,8 +408,16 @@ def bench_serve(seconds=10.0, rate=50.0, ce_scale=0.01, nce_scale=0.0002, nce_ma
         span = max(i["t_end"] for i in binf) - min(i["t_submit"] for i in binf)
         return sum(j["R"] * j["steps"] for j in ce_jobs) / span, span
     burst(8)                                               # warm-up: kernels loaded, pools grown
-    cap = {w: burst(w) for w in (8, 16, 32)}               # the launch shape of the served CE rounds
-    w_best = max(cap, key=lambda w: cap[w][0])
+    # the launch shape of the served CE rounds: the windowed kernel has its own, so its bursts only show the spread from run to
+    # run (the middle one is reported); a set without window tables takes the best of three
+    own_shape = all(chunk_kernel([m], None, 32)[0] == "windowed" for m in {id(j["model"]): j["model"] for j in ce_jobs}.values())
+    if own_shape:
+        runs = sorted(burst(8) for _ in range(3))
+        cap, w_best, best = {8: runs[1]}, 8, runs[1]
+    else:
+        cap = {w: burst(w) for w in (8, 16, 32)}
+        w_best = max(cap, key=lambda w: cap[w][0])
+        runs, best = [cap[w] for w in cap], cap[w_best]
     srv = Server(precision=32, warps=w_best)
     hs = []
     start = time.perf_counter()
@@ -410,7 +442,7 @@ def bench_serve(seconds=10.0, rate=50.0, ce_scale=0.01, nce_scale=0.0002, nce_ma
     att = {k: sum(j["R"] * j["steps"] for j in jobs if j["kind"] == k) for k in ("ce", "nce")}
     # capacity (above): every CE job of the stream submitted at once; against each alone, one after another, in the
     # plain float64 kernel (general point-function products), chunks of the same exchange interval
-    burst_s = cap[w_best][1]
+    burst_s = best[1]
     a_att, a_s = 0, 0.0
     for j in ce_jobs[:alone_jobs] if alone_jobs else ce_jobs:
         gce = j["model"]
@@ -440,7 +472,8 @@ def bench_serve(seconds=10.0, rate=50.0, ce_scale=0.01, nce_scale=0.0002, nce_ma
             "makespan_s": makespan, "attempts": st["attempts"], "attempts_ce": att["ce"], "attempts_nce": att["nce"],
             "ce_attempts_per_s_poisson": ce_rate,
             "ce_capacity_attempts_per_s": att["ce"] / burst_s, "ce_capacity_makespan_s": burst_s,
-            "ce_warps": w_best, "ce_capacity_by_warps": {str(w): v[0] for w, v in cap.items()},
+            "ce_kernel": "windowed" if own_shape else f"{w_best} warps", "ce_capacity_runs": [round(v[0]) for v in runs],
+            "ce_capacity_of": "middle of three runs" if own_shape else "best of 8, 16 and 32 warps",
             "fp64_single_job_alone": (a_att / a_s) if a_s else None,
             "ratio_ce_capacity_vs_fp64_alone": (att["ce"] / burst_s) / (a_att / a_s) if a_s else None,
             "rounds": {"ce": st["rounds_ce"], "nce": st["rounds_nce"]}, "setup_s": setup}
@@ -454,7 +487,7 @@ def bench_large(L=136, R=256, chunk=5000, steps=3, warmup=1, precision=64, seed=
     chunk of ``chunk`` MC steps per replica + exchange + re-anchor."""
     import torch
     from neuralce_gb300.autotune import best_launch
-    from neuralce_gb300.pt import PTState, run_chunk
+    from neuralce_gb300.pt import PTState, chunk_kernel, run_chunk
     from neuralce_gb300.workloads import ServeModels, ladder
     t0 = time.time()
     gce = ServeModels().ce(L)
@@ -481,6 +514,7 @@ def bench_large(L=136, R=256, chunk=5000, steps=3, warmup=1, precision=64, seed=
         a_, b_ = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a_.record(); st.enable_field(gce); b_.record(); torch.cuda.synchronize()
         field_ms = a_.elapsed_time(b_)
+    kernel, threads = chunk_kernel([gce], [st], precision, path)
     step = 0
     from neuralce_gb300 import _lib
 
@@ -509,20 +543,21 @@ def bench_large(L=136, R=256, chunk=5000, steps=3, warmup=1, precision=64, seed=
     a_, b_ = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     a_.record(); gce.batched_energy(st.sigma); b_.record(); torch.cuda.synchronize()
     hbm, src = peaks()
-    achieved = value * B_GATHER / 1e9
+    need = ce_chunk_bytes(gce, kernel, R, chunk)
+    achieved = need / (tot / steps) / 1e9
     return {"value": value, "unit": "swap attempts/s", "ms_per_step": float(np.mean(ms)),
             "config": f"CE large cell: fcc {L}^3 conventional ({N} sites), R={R} 300-1400 K, "
-                      f"{'local-field' if path == 3 else 'sign-parity'} kernel, fp{precision} (exact fixed point) dE, "
+                      f"{kernel} kernel, fp{precision} (exact fixed point) dE, "
                       f"chunk {chunk} steps + fp64 exchange + exact fp64 re-anchor from cluster-vector sums",
-            "sites": N, "replicas": R, "state_bytes": R * N * (9 if path == 3 else 1), "warps_per_replica": w,
+            "sites": N, "replicas": R, "state_bytes": R * N * (9 if path == 3 else 1), "launch": ce_launch(kernel, threads, w, 1),
             "path": {2: "sign-parity", 3: "local-field"}[path], "autotune_ms": {str(k): round(v, 3) for k, v in tune.items()},
             "tracked_sums_equal_recount": cv_ok, "fields_equal_rebuild": field_ok,
             "max_E_vs_full_recompute_eV": float((Ef - st.E).abs().max().item()), "field_init_ms": field_ms,
             "full_energy_ms": a_.elapsed_time(b_), "full_energy_site_replicas_per_s": R * N / (a_.elapsed_time(b_) / 1e3),
             "accept_rate": float(st.n_acc.sum().item()) / (R * step),
             "near_threshold_steps": int(st.n_near.sum().item()),
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-                         "peak_source": src, "bytes_per_attempt": B_GATHER},
+            "roofline": {"bound": "latency" if kernel == "windowed" else "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
+                         "frac": achieved / hbm, "peak_source": src, "algorithmic_bytes_per_launch": need},
             "setup_s": setup, "tables_s": setup_tables, "vs_h100_published_4344547": value / 4_344_547}
 
 
@@ -680,7 +715,7 @@ def main():
         import torch.distributed as dist
         dist.init_process_group("nccl")
     from neuralce_gb300 import _lib
-    from neuralce_gb300.pt import PTState, run_chunk, make_chunk
+    from neuralce_gb300.pt import PTState, chunk_kernel, run_chunk, make_chunk
     from neuralce_gb300.workloads import ce_config, ladder, replica_configs
     _lib.lib()
     gce, sig = ce_config(args.L, seed=rank)
@@ -700,6 +735,7 @@ def main():
         tuned = {f"{w}x{c}/p{p}": round(v, 3) for (w, c, p), v in t.items()}
     if args.path == 3:
         st.enable_field(gce)                               # local fields of the replicas' occupancies
+    kernel, threads = chunk_kernel([gce], [st], args.precision, args.path)
     si = 100                                               # energy samples every 100 steps (the CLI default)
     Es = torch.zeros((T // si, R), dtype=torch.float64, device="cuda")
     flush = torch.empty(256 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
@@ -759,17 +795,14 @@ def main():
                "d2h_bytes_per_step": d2h, "api": "nce_ce_run_chunk_host"}
     hbm, src = peaks()
     ms_chunk = float(np.mean(per_ms))
-    achieved = R * T * B_GATHER / (ms_chunk / 1e3) / 1e9
-    # DRAM bytes per launch from one ncu capture of this workload (dram__bytes_read.sum + dram__bytes_write.sum of
-    # ce_win_chunk_kernel, 2,048 sites, R = 32): the tables live in shared memory, the occupancies in the L1 and L2;
-    # the same capture's shared-memory pipe use (l1tex__data_pipe_lsu_wavefronts_mem_shared.sum.pct_of_peak_sustained
-    # _elapsed), the on-chip roofline that the gathered bytes actually meet
-    traffic = TRAFFIC.get((args.path, args.L, args.R, T))
-    roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm, "traffic": traffic,
-            "kernel": {1: "ce_pt_chunk_kernel", 3: "ce_lf_chunk_kernel"}.get(args.path, "ce_win_chunk_kernel"),
-            "peak_source": src,
-            "algorithmic_bytes_per_launch": R * T * B_GATHER,
-            "shared_pipe_frac_ncu": SMEM_PIPE.get((args.path, args.L, args.R, T))}
+    need = ce_chunk_bytes(gce, kernel, R, T)
+    achieved = need / (ms_chunk / 1e3) / 1e9
+    # windowed: neither memory nor a math pipe bounds it (the tables and occupancies stay on chip and in L2; `traffic` is the
+    # DRAM bytes of a launch, shared_pipe_frac_ncu the shared-memory wavefronts, both from the capture above)
+    roof = {"bound": "latency" if kernel == "windowed" else "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
+            "frac": achieved / hbm, "traffic": TRAFFIC.get((kernel, args.L, args.R)), "kernel": CE_KERNELS[kernel],
+            "peak_source": src, "algorithmic_bytes_per_launch": need,
+            "shared_pipe_frac_ncu": SMEM_PIPE.get((kernel, args.L, args.R))}
     nce_line = nce_tc_line = nce_bf16_line = nce_shipped_line = None
     if rank == 0 and args.nce_steps > 0:
         nce_line = bench_nce(steps=args.nce_steps)
@@ -800,7 +833,7 @@ def main():
                 "config": workload_config(args, gce), "clocks": clocks, "e2e": e2e, "gpu_launches": args.steps,
                 "roofline": roof, "cpu_baseline": cpu, "nce": nce_line, "nce_tcgen05_split": nce_tc_line, "nce_tcgen05_bf16": nce_bf16_line, "nce_shipped_model": nce_shipped_line, "batch": batch_line, "serve": serve_line,
                 "large_ce": large_ce_line, "large_nce": large_nce_line,
-                "launch": {"warps_per_cta": args.warps, "ctas_per_replica": args.cluster,
+                "launch": {**ce_launch(kernel, threads, args.warps, args.cluster),
                            "path": ["auto", "general", "sign-parity", "local-field"][args.path],
                            "autotune_ms": tuned},
                 "accept_rate": float(st.n_acc.sum().item()) / max(1, R * step),
