@@ -540,8 +540,8 @@ __device__ void layer_tiles(const NceJob &jb, int lvl, const LayerW &LW, const f
             using V4 = std::integral_constant<int, 4>; using V2 = std::integral_constant<int, 2>; using V1 = std::integral_constant<int, 1>;
             // (layer-0 rows come from the caller's buffer, which any float alignment may start: loads as wide as both the
             // row length and the address allow; the step's new rows and the zero row start on 16 bytes)
-            const uintptr_t at = reinterpret_cast<uintptr_t>(cache);
-            const bool by4 = (Cin & 3) == 0 && (at & 15) == 0, by2 = (Cin & 1) == 0 && (at & 7) == 0;
+            const uint32_t at = (uint32_t)reinterpret_cast<uintptr_t>(cache) | (uint32_t)(Cin * 4);   // bytes: where every row starts
+            const bool by4 = (at & 15) == 0, by2 = (at & 7) == 0;
             if (m.tc_split) {
                 if (by4) gather(V4{}, std::true_type{});
                 else if (by2) gather(V2{}, std::true_type{});
